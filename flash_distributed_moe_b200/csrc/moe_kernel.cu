@@ -301,6 +301,17 @@ __device__ __forceinline__ bool wait_bar(const FdmoeParams& p, SmemCtl& sc, uint
   return true;
 }
 
+// The same wait by a whole warp: every lane polls, all lanes take the same decision.  The TMA and MMA
+// warps run their loops warp-wide and let one elected lane issue: inside a branch on the lane index the
+// compiler cannot tell that a single thread is active, and every tcgen05 and TMA instruction, whose
+// operands must be warp-uniform, then costs several times its issue time.  Measured on the MMA warp's
+// wait-issue-commit loop alone: 461 cycles per k-block at any tile width under `lane == 0`, 277 at N = 32
+// and 299 at N = 128 with an elected lane of a converged warp (the tensor pipe needs 256 at N = 128, 512 at 256).
+__device__ __forceinline__ bool wait_bar_warp(const FdmoeParams& p, SmemCtl& sc, uint64_t* bar, uint32_t parity,
+                                              uint32_t err_code, uint32_t budgets = 1u) {
+  return __all_sync(0xffffffffu, wait_bar(p, sc, bar, parity, err_code, budgets));
+}
+
 // Same wait without raising an error: one budget's worth of polling.
 __device__ __forceinline__ bool wait_idle(const FdmoeParams& p, SmemCtl& sc, uint64_t* bar, uint32_t parity) {
   const uint64_t t0 = ptx::globaltimer_ns();
@@ -1341,11 +1352,12 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
     }
     __syncwarp();
   } else if (warp == kWarpTma) {
-    if (lane == 0) {
+    {
+      const bool elected = ptx::elect_one();
       uint32_t stage_it = 0;
       for (uint32_t it = 0;; ++it) {
         const uint32_t r = it % kRing, ph = (it / kRing) & 1u;
-        if (!wait_bar(p, sc, &sc.ring_full[r], ph, FDMOE_ERR_TIMEOUT_RING, 2u)) break;
+        if (!wait_bar_warp(p, sc, &sc.ring_full[r], ph, FDMOE_ERR_TIMEOUT_RING, 2u)) break;
         const FdmoeSlot t = sc.ring[r];
         const uint32_t kind = t.a & 0xffu;
         if (kind == FDMOE_TASK_EXIT) break;
@@ -1363,27 +1375,30 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           bool ok = true;
           for (uint32_t kb = 0; kb < nkb && ok; kb += gk, ++stage_it) {
             const uint32_t s = stage_it % kStages, sph = (stage_it / kStages) & 1u;
-            ok = wait_bar(p, sc, &sc.empty_bar[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
+            ok = wait_bar_warp(p, sc, &sc.empty_bar[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
             if (!ok) break;
             uint8_t* sa = stage + s * kStageBytes;
             uint8_t* sb = sa + kStageA;
-            ptx::mbar_expect_tx(&sc.full_bar[s], gt ? gk * gate_bytes : (uint32_t)kStageBytes);
-            const int32_t kx = (int32_t)(kb * FDMOE_TILE_K);
-            if (gt) {
-              for (uint32_t i = 0; i < gk; ++i) {
-                ptx::tma_load_2d(sa + i * (kStageA / 2), &p.tm_x, &sc.full_bar[s], kx + (int32_t)(i * FDMOE_TILE_K), arow);
-                ptx::tma_load_2d(sb + i * kStageA, &p.tm_gate, &sc.full_bar[s], kx + (int32_t)(i * FDMOE_TILE_K), 0);
+            if (elected) {
+              ptx::mbar_expect_tx(&sc.full_bar[s], gt ? gk * gate_bytes : (uint32_t)kStageBytes);
+              const int32_t kx = (int32_t)(kb * FDMOE_TILE_K);
+              if (gt) {
+                for (uint32_t i = 0; i < gk; ++i) {
+                  ptx::tma_load_2d(sa + i * (kStageA / 2), &p.tm_x, &sc.full_bar[s], kx + (int32_t)(i * FDMOE_TILE_K), arow);
+                  ptx::tma_load_2d(sb + i * kStageA, &p.tm_gate, &sc.full_bar[s], kx + (int32_t)(i * FDMOE_TILE_K), 0);
+                }
+              } else if (f1) {
+                ptx::tma_load_2d(sa, &p.tm_packed, &sc.full_bar[s], kx, arow);
+                const int32_t brow = (int32_t)(e * 2u * (uint32_t)p.I + n * FDMOE_TILE_N1);
+                ptx::tma_load_2d(sb, &p.tm_w13, &sc.full_bar[s], kx, brow);
+                ptx::tma_load_2d(sb + kStageA, &p.tm_w13, &sc.full_bar[s], kx, brow + p.I);
+              } else {
+                ptx::tma_load_2d(sa, &p.tm_act, &sc.full_bar[s], kx, arow);
+                const int32_t brow = (int32_t)(e * (uint32_t)p.H + n * FDMOE_TILE_N2);
+                ptx::tma_load_2d(sb, &p.tm_w2, &sc.full_bar[s], kx, brow);
               }
-            } else if (f1) {
-              ptx::tma_load_2d(sa, &p.tm_packed, &sc.full_bar[s], kx, arow);
-              const int32_t brow = (int32_t)(e * 2u * (uint32_t)p.I + n * FDMOE_TILE_N1);
-              ptx::tma_load_2d(sb, &p.tm_w13, &sc.full_bar[s], kx, brow);
-              ptx::tma_load_2d(sb + kStageA, &p.tm_w13, &sc.full_bar[s], kx, brow + p.I);
-            } else {
-              ptx::tma_load_2d(sa, &p.tm_act, &sc.full_bar[s], kx, arow);
-              const int32_t brow = (int32_t)(e * (uint32_t)p.H + n * FDMOE_TILE_N2);
-              ptx::tma_load_2d(sb, &p.tm_w2, &sc.full_bar[s], kx, brow);
             }
+            __syncwarp();
           }
           if (!ok) break;
         } else if (kind == FDMOE_TASK_DISPATCH) {
@@ -1394,25 +1409,31 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           bool ok = true;
           for (uint32_t r0 = 0; r0 < nt && ok; r0 += rps, ++stage_it) {
             const uint32_t s = stage_it % kStages, sph = (stage_it / kStages) & 1u;
-            ok = wait_bar(p, sc, &sc.empty_bar[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
+            ok = wait_bar_warp(p, sc, &sc.empty_bar[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
             if (!ok) break;
             const uint32_t bytes = min(rps, nt - r0) * rowb;
-            ptx::mbar_expect_tx(&sc.full_bar[s], bytes);
-            ptx::bulk_load_1d(stage + s * kStageBytes, xb + (size_t)r0 * rowb, bytes, &sc.full_bar[s]);
+            if (elected) {
+              ptx::mbar_expect_tx(&sc.full_bar[s], bytes);
+              ptx::bulk_load_1d(stage + s * kStageBytes, xb + (size_t)r0 * rowb, bytes, &sc.full_bar[s]);
+            }
+            __syncwarp();
           }
           if (!ok) break;
         } else if (kind == FDMOE_TASK_GATEFIX) {
           bool ok = true;
           for (uint32_t kb = 0; kb < nkb1; kb += kFixBlocks, ++stage_it) {
             const uint32_t s = stage_it % kStages, sph = (stage_it / kStages) & 1u;
-            ok = wait_bar(p, sc, &sc.empty_bar[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
+            ok = wait_bar_warp(p, sc, &sc.empty_bar[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
             if (!ok) break;
             const uint32_t nb = min((uint32_t)kFixBlocks, nkb1 - kb);
             const uint32_t blk_bytes = (uint32_t)min(128, p.E) * FDMOE_TILE_K * 2u;
-            ptx::mbar_expect_tx(&sc.full_bar[s], nb * blk_bytes);
-            for (uint32_t i = 0; i < nb; ++i)
-              ptx::tma_load_2d(stage + s * kStageBytes + i * kStageA, &p.tm_gate, &sc.full_bar[s],
-                               (int32_t)((kb + i) * FDMOE_TILE_K), 0);
+            if (elected) {
+              ptx::mbar_expect_tx(&sc.full_bar[s], nb * blk_bytes);
+              for (uint32_t i = 0; i < nb; ++i)
+                ptx::tma_load_2d(stage + s * kStageBytes + i * kStageA, &p.tm_gate, &sc.full_bar[s],
+                                 (int32_t)((kb + i) * FDMOE_TILE_K), 0);
+            }
+            __syncwarp();
           }
           if (!ok) break;
         } else if (kind == FDMOE_TASK_COMBINE) {
@@ -1423,34 +1444,39 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           for (int tk = t_begin; tk < t_end && ok; ++tk) {
             for (int c0 = 0; c0 < p.H; c0 += kCombineCols, ++stage_it) {
               const uint32_t s = stage_it % kStages, sph = (stage_it / kStages) & 1u;
-              ok = wait_bar(p, sc, &sc.empty_bar[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
+              ok = wait_bar_warp(p, sc, &sc.empty_bar[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
               if (!ok) break;
               const uint32_t wbytes = (uint32_t)min(kCombineCols, p.H - c0) * 2u;
               uint8_t* sa = stage + s * kStageBytes;
-              ptx::mbar_expect_tx(&sc.full_bar[s], wbytes * (uint32_t)p.K);
-              if (p.H <= kCombineCols) {
-                // the K rows of a token are contiguous: one copy
-                ptx::bulk_load_1d(sa, ys + (size_t)tk * p.K * p.H, wbytes * (uint32_t)p.K, &sc.full_bar[s]);
-              } else {
-                for (int k = 0; k < p.K; ++k)
-                  ptx::bulk_load_1d(sa + k * wbytes, ys + ((size_t)tk * p.K + k) * p.H + c0, wbytes, &sc.full_bar[s]);
+              if (elected) {
+                ptx::mbar_expect_tx(&sc.full_bar[s], wbytes * (uint32_t)p.K);
+                if (p.H <= kCombineCols) {
+                  // the K rows of a token are contiguous: one copy
+                  ptx::bulk_load_1d(sa, ys + (size_t)tk * p.K * p.H, wbytes * (uint32_t)p.K, &sc.full_bar[s]);
+                } else {
+                  for (int k = 0; k < p.K; ++k)
+                    ptx::bulk_load_1d(sa + k * wbytes, ys + ((size_t)tk * p.K + k) * p.H + c0, wbytes, &sc.full_bar[s]);
+                }
               }
+              __syncwarp();
             }
           }
           if (!ok) break;
         }
-        ptx::mbar_arrive(&sc.ring_empty[r]);
+        __syncwarp();  // every lane has read the slot
+        if (elected) ptx::mbar_arrive(&sc.ring_empty[r]);
       }
     }
     __syncwarp();
   } else if (warp == kWarpMma) {
-    if (lane == 0) {
+    {
+      const bool elected = ptx::elect_one();
       constexpr uint32_t idesc256 = ptx::make_idesc_bf16(128, 256);
       constexpr uint32_t idesc128 = ptx::make_idesc_bf16(128, 128);
       uint32_t stage_it = 0, tile_it = 0, skips = 0;
       for (uint32_t it = 0;; ++it) {
         const uint32_t r = it % kRing, ph = (it / kRing) & 1u;
-        if (!wait_bar(p, sc, &sc.ring_full[r], ph, FDMOE_ERR_TIMEOUT_RING, 2u)) break;
+        if (!wait_bar_warp(p, sc, &sc.ring_full[r], ph, FDMOE_ERR_TIMEOUT_RING, 2u)) break;
         const FdmoeSlot t = sc.ring[r];
         const uint32_t kind = t.a & 0xffu;
         if (kind == FDMOE_TASK_EXIT) break;
@@ -1460,30 +1486,33 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           const uint32_t idesc = (kind == FDMOE_TASK_GATE) ? idesc128 : idesc256;
           const uint32_t acc = tile_it & 1u, aph = (tile_it >> 1) & 1u;
           ++tile_it;
-          if (!wait_bar(p, sc, &sc.tmem_empty[acc], aph ^ 1u, FDMOE_ERR_TIMEOUT_TMEM)) break;
+          if (!wait_bar_warp(p, sc, &sc.tmem_empty[acc], aph ^ 1u, FDMOE_ERR_TIMEOUT_TMEM)) break;
           ptx::tcgen05_fence_after();
           const uint32_t d_tmem = tmem_base + acc * kAccCols;
           const uint32_t gk = gate_kblocks_per_stage(kind == FDMOE_TASK_GATE, p.gate_rows);
           for (uint32_t kb = 0; kb < nkb; kb += gk, ++stage_it) {
             const uint32_t s = stage_it % kStages, sph = (stage_it / kStages) & 1u;
-            ok = wait_bar(p, sc, &sc.full_bar[s], sph, FDMOE_ERR_TIMEOUT_STAGE);
+            ok = wait_bar_warp(p, sc, &sc.full_bar[s], sph, FDMOE_ERR_TIMEOUT_STAGE);
             if (!ok) break;
             ptx::tcgen05_fence_after();
-            const uint32_t sa = ptx::smem_u32(stage + s * kStageBytes);
-            for (uint32_t i = 0; i < gk; ++i) {
-              // (a GATE stage with two k-blocks: A at 8 KB, B at 16 KB steps)
-              const uint64_t da = ptx::make_smem_desc_sw128(sa + i * (kStageA / 2));
-              const uint64_t db = ptx::make_smem_desc_sw128(sa + kStageA + i * kStageA);
+            if (elected) {
+              const uint32_t sa = ptx::smem_u32(stage + s * kStageBytes);
+              for (uint32_t i = 0; i < gk; ++i) {
+                // (a GATE stage with two k-blocks: A at 8 KB, B at 16 KB steps)
+                const uint64_t da = ptx::make_smem_desc_sw128(sa + i * (kStageA / 2));
+                const uint64_t db = ptx::make_smem_desc_sw128(sa + kStageA + i * kStageA);
 #pragma unroll
-              for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4) {
-                // +32 bytes per 16-element k step inside the 128-byte swizzle row
-                ptx::umma_bf16(d_tmem, da + k4 * 2u, db + k4 * 2u, idesc, (kb | i | k4) != 0u);
+                for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4) {
+                  // +32 bytes per 16-element k step inside the 128-byte swizzle row
+                  ptx::umma_bf16(d_tmem, da + k4 * 2u, db + k4 * 2u, idesc, (kb | i | k4) != 0u);
+                }
               }
+              ptx::umma_commit(&sc.empty_bar[s]);  // frees the stage when the MMAs have read it
             }
-            ptx::umma_commit(&sc.empty_bar[s]);  // frees the stage when the MMAs have read it
+            __syncwarp();
           }
           if (!ok) break;
-          ptx::umma_commit(&sc.tmem_full[acc]);
+          if (elected) ptx::umma_commit(&sc.tmem_full[acc]);
         }
         if (kind == FDMOE_TASK_DISPATCH || kind == FDMOE_TASK_GATEFIX || kind == FDMOE_TASK_COMBINE) {
           // Stages of these tasks are consumed
@@ -1504,6 +1533,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
               __nanosleep(100);
             }
           }
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           if (kind == FDMOE_TASK_DISPATCH) {
             stage_it += dispatch_stages(p, t.c);
@@ -1513,7 +1543,8 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
             stage_it += t.c * (uint32_t)((p.H + kCombineCols - 1) / kCombineCols);
           }
         }
-        ptx::mbar_arrive(&sc.ring_empty[r]);
+        __syncwarp();  // every lane has read the slot
+        if (elected) ptx::mbar_arrive(&sc.ring_empty[r]);
       }
     }
     __syncwarp();
