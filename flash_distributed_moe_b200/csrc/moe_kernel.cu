@@ -53,6 +53,11 @@ constexpr int kStages = 4;
 constexpr int kStageA = FDMOE_TILE_M * FDMOE_TILE_K * 2;  // 16 KB
 constexpr int kStageB = 256 * FDMOE_TILE_K * 2;           // 32 KB
 constexpr int kStageBytes = kStageA + kStageB;            // 48 KB
+// Wide stages, for FFN tiles of an expert with more than 128 rows: two 128-row blocks of rows against
+// one 256-row block of weights.  They lie over the same shared memory as the narrow ones.
+constexpr int kWideStages = 3;
+constexpr int kWideBytes = 2 * kStageA + kStageB;  // 64 KB
+static_assert(kWideStages * kWideBytes <= kStages * kStageBytes, "wide stages share the narrow stages' memory");
 constexpr int kRing = 3;
 constexpr int kFixBlocks = 3;  // k-blocks of gate weights per stage in a GATEFIX task (3 x 16 KB)
 constexpr int kDone = 8;  // depth of the hand-off ring to the completion warp
@@ -62,6 +67,8 @@ constexpr int kAccCols = 256;
 struct __align__(64) SmemCtl {
   uint64_t full_bar[kStages];
   uint64_t empty_bar[kStages];
+  uint64_t wide_full[kWideStages];
+  uint64_t wide_empty[kWideStages];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint64_t ring_full[kRing];
@@ -1046,7 +1053,9 @@ __device__ __noinline__ void gated_task(const FdmoeParams& p, SmemCtl& sc, int e
     ntile = (lcnt + 127u) / 128u;
     first = ((lcnt / 128u) / B) * B;
   }
-  const uint32_t mytasks = (ntile - first) * nt1;
+  // m-tiles per task (see FDMOE_TILE_WIDE for the reason of the line at 128 rows)
+  const uint32_t step = (!S && lcnt > 128u) ? 2u : 1u;
+  const uint32_t mytasks = ((ntile - first + step - 1u) / step) * nt1;
   uint32_t inc = mytasks, inc_tile = ntile;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
@@ -1076,14 +1085,13 @@ __device__ __noinline__ void gated_task(const FdmoeParams& p, SmemCtl& sc, int e
   epi_bar();
   if (mytasks) {
     const uint32_t t1 = sc.q_t0 + before + inc - mytasks;
-    const uint32_t full = lcnt / 128u, rem = lcnt % 128u;
     FdmoeSlot* slots = me.slots[1];
     for (uint32_t idx = 0; idx < mytasks; ++idx) {
-      const uint32_t jt = first + idx / nt1, n = idx % nt1;
+      const uint32_t jt = first + (idx / nt1) * step, n = idx % nt1;
       FdmoeSlot* sl = &slots[(t1 + idx) & (uint32_t)p.queue_mask];
       sl->a = task_word(FDMOE_TASK_FFN1, (uint32_t)etid, n);
       sl->b = jt;
-      sl->c = (jt < full) ? 128u : rem;
+      sl->c = min(128u * step, lcnt - jt * 128u) | (step > 1u ? (uint32_t)FDMOE_TILE_WIDE : 0u);
     }
     fence_acqrel<false>();
     for (uint32_t idx = 0; idx < mytasks; ++idx)
@@ -1132,10 +1140,19 @@ __device__ __forceinline__ void store_staged_rows(uint8_t* st, int lane, unsigne
   __syncwarp();
 }
 
-// FFN1 epilogue: act[row, n*128 + c] = silu(D[row, c]) * D[row, 128 + c].
-__device__ __forceinline__ void ffn1_epilogue(const FdmoeParams& p, SmemCtl& sc, uint32_t taddr, int q, int h,
-                                              int lane, int ewarp, uint32_t e, uint32_t j, uint32_t n,
-                                              uint32_t rows) {
+// This warp has read its part of an accumulator: the MMA warp may overwrite it once all have.
+__device__ __forceinline__ void release_acc(uint64_t* tmem_empty_bar, int lane) {
+  ptx::tcgen05_fence_before();
+  __syncwarp();
+  if (lane == 0) ptx::mbar_arrive(tmem_empty_bar);
+}
+
+// FFN1 epilogue: act[row, n*128 + c] = silu(D[row, c]) * D[row, 128 + c].  Both epilogues bring their
+// whole part of the accumulator into registers first and release it before they compute and store: a
+// wide task fills both accumulators, so the next task's MMAs wait for nothing else.
+__device__ __forceinline__ void ffn1_epilogue(const FdmoeParams& p, SmemCtl& sc, uint32_t taddr,
+                                              uint64_t* tmem_empty_bar, int q, int h, int lane, int ewarp, uint32_t e,
+                                              uint32_t j, uint32_t n, uint32_t rows) {
   uint8_t* st = sc.store_stage[ewarp];
   const uint32_t row = q * 32 + lane;
   unsigned long long myptr = 0ull;
@@ -1144,55 +1161,70 @@ __device__ __forceinline__ void ffn1_epilogue(const FdmoeParams& p, SmemCtl& sc,
                                                  ((size_t)e * p.cap_rows + (size_t)j * 128 + row) * p.I +
                                                  n * FDMOE_TILE_N1 + h * 64);
   const uint32_t tbase = taddr + ((uint32_t)(q * 32) << 16) + h * 64;
+  uint32_t g[2][32], u[2][32];
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    uint32_t g[32], u[32], o[16];
-    ptx::tmem_ld_32x32(tbase + c * 32, g);
-    ptx::tmem_ld_32x32(tbase + 128 + c * 32, u);
-    ptx::tmem_ld_wait();
+    ptx::tmem_ld_32x32(tbase + c * 32, g[c]);
+    ptx::tmem_ld_32x32(tbase + 128 + c * 32, u[c]);
+  }
+  ptx::tmem_ld_wait();
+  release_acc(tmem_empty_bar, lane);
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint32_t o[16];
 #pragma unroll
     for (int w = 0; w < 16; ++w)
-      o[w] = pack_bf16(silu_mul(__uint_as_float(g[2 * w]), __uint_as_float(u[2 * w])),
-                       silu_mul(__uint_as_float(g[2 * w + 1]), __uint_as_float(u[2 * w + 1])));
+      o[w] = pack_bf16(silu_mul(__uint_as_float(g[c][2 * w]), __uint_as_float(u[c][2 * w])),
+                       silu_mul(__uint_as_float(g[c][2 * w + 1]), __uint_as_float(u[c][2 * w + 1])));
     stage_half_row(st, lane, c, o);
   }
   store_staged_rows(st, lane, myptr);
 }
 
-// FFN2 epilogue: y[token, slot, n*256 + c] = D[row, c] * routing weight, stored
-// on the token's home rank.  Returns whether this thread's row went to another GPU.
-__device__ __forceinline__ bool ffn2_epilogue(const FdmoeParams& p, SmemCtl& sc, uint32_t taddr, int q, int h,
-                                              int lane, int ewarp, uint32_t e, uint32_t j, uint32_t n,
-                                              uint32_t rows) {
-  uint8_t* st = sc.store_stage[ewarp];
+// Where an FFN2 tile's row goes: y[token, slot] on the token's home rank.
+struct YRow {
+  unsigned long long ptr;  // first byte of this thread's 128 columns, 0 = no row
+  float weight;
+  bool remote;             // the row goes to another GPU
+};
+__device__ __forceinline__ YRow ffn2_row(const FdmoeParams& p, int q, int h, int lane, uint32_t e, uint32_t j,
+                                         uint32_t n, uint32_t rows) {
+  YRow y{0ull, 0.f, false};
   const uint32_t row = q * 32 + lane;
-  float wgt = 0.f;
-  unsigned long long myptr = 0ull;
-  bool remote = false;
   if (row < rows) {
     const uint4 mraw = ld_cg_u4(&p.peers[p.rank].meta[(size_t)e * p.cap_rows + (size_t)j * 128 + row]);
     const int token = (int)mraw.x, home = (int)mraw.y >> 8, slot = (int)mraw.y & 0xff;
-    wgt = __uint_as_float(mraw.z);
-    remote = home != p.rank;
-    myptr = reinterpret_cast<unsigned long long>(reinterpret_cast<bf16*>(p.peers[home].ystage) +
+    y.weight = __uint_as_float(mraw.z);
+    y.remote = home != p.rank;
+    y.ptr = reinterpret_cast<unsigned long long>(reinterpret_cast<bf16*>(p.peers[home].ystage) +
                                                  ((size_t)token * p.K + slot) * p.H + n * FDMOE_TILE_N2 + h * 128);
   }
+  return y;
+}
+
+// FFN2 epilogue: y[token, slot, n*256 + c] = D[row, c] * routing weight, stored on the token's home rank.
+__device__ __forceinline__ void ffn2_epilogue(SmemCtl& sc, uint32_t taddr, uint64_t* tmem_empty_bar, int q, int h,
+                                              int lane, int ewarp, const YRow& y) {
+  uint8_t* st = sc.store_stage[ewarp];
   const uint32_t tbase = taddr + ((uint32_t)(q * 32) << 16) + h * 128;
+  uint32_t d[4][32];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32(tbase + c * 32, d[c]);
+  ptx::tmem_ld_wait();
+  release_acc(tmem_empty_bar, lane);
 #pragma unroll
   for (int pass = 0; pass < 2; ++pass) {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      uint32_t d[32], o[16];
-      ptx::tmem_ld_32x32(tbase + (pass * 2 + c) * 32, d);
-      ptx::tmem_ld_wait();
+      uint32_t o[16];
 #pragma unroll
       for (int w = 0; w < 16; ++w)
-        o[w] = pack_bf16(__uint_as_float(d[2 * w]) * wgt, __uint_as_float(d[2 * w + 1]) * wgt);
+        o[w] = pack_bf16(__uint_as_float(d[pass * 2 + c][2 * w]) * y.weight,
+                         __uint_as_float(d[pass * 2 + c][2 * w + 1]) * y.weight);
       stage_half_row(st, lane, c, o);
     }
-    store_staged_rows(st, lane, myptr ? myptr + (unsigned long long)(pass * 128) : 0ull);
+    store_staged_rows(st, lane, y.ptr ? y.ptr + (unsigned long long)(pass * 128) : 0ull);
   }
-  return remote;
 }
 
 // COMBINE streams the K weighted rows of each token of a group through the
@@ -1245,6 +1277,10 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&sc.full_bar[s], 1);
       ptx::mbar_init(&sc.empty_bar[s], 1);
+    }
+    for (int s = 0; s < kWideStages; ++s) {
+      ptx::mbar_init(&sc.wide_full[s], 1);
+      ptx::mbar_init(&sc.wide_empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(&sc.tmem_full[a], 1);
@@ -1354,13 +1390,65 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
   } else if (warp == kWarpTma) {
     {
       const bool elected = ptx::elect_one();
-      uint32_t stage_it = 0;
+      uint32_t stage_it = 0, wide_it = 0;
+      bool wide_now = false;
       for (uint32_t it = 0;; ++it) {
         const uint32_t r = it % kRing, ph = (it / kRing) & 1u;
         if (!wait_bar_warp(p, sc, &sc.ring_full[r], ph, FDMOE_ERR_TIMEOUT_RING, 2u)) break;
         const FdmoeSlot t = sc.ring[r];
         const uint32_t kind = t.a & 0xffu;
         if (kind == FDMOE_TASK_EXIT) break;
+        const bool wide = (kind == FDMOE_TASK_FFN1 || kind == FDMOE_TASK_FFN2) && (t.c & FDMOE_TILE_WIDE) != 0u;
+        const bool staged = kind == FDMOE_TASK_FFN1 || kind == FDMOE_TASK_FFN2 || kind == FDMOE_TASK_GATE ||
+                            kind == FDMOE_TASK_DISPATCH || kind == FDMOE_TASK_GATEFIX || kind == FDMOE_TASK_COMBINE;
+        if (staged && wide != wide_now) {
+          // narrow and wide stages lie over the same memory: every stage filled so far has to be free
+          // (use u of a stage ends phase u / stages of its barrier)
+          bool drained = true;
+          if (wide) {
+            for (uint32_t u = stage_it > kStages ? stage_it - kStages : 0u; u < stage_it && drained; ++u)
+              drained = wait_bar_warp(p, sc, &sc.empty_bar[u % kStages], (u / kStages) & 1u, FDMOE_ERR_TIMEOUT_STAGE);
+          } else {
+            for (uint32_t u = wide_it > kWideStages ? wide_it - kWideStages : 0u; u < wide_it && drained; ++u)
+              drained = wait_bar_warp(p, sc, &sc.wide_empty[u % kWideStages], (u / kWideStages) & 1u,
+                                      FDMOE_ERR_TIMEOUT_STAGE);
+          }
+          if (!drained) break;
+          wide_now = wide;
+        }
+        if (wide) {
+          const uint32_t e = (t.a >> 8) & 0xfffu, n = t.a >> 20, rows = t.c & FDMOE_TILE_ROWS;
+          const bool f1 = kind == FDMOE_TASK_FFN1, pair = rows > 128u;
+          const uint32_t nkb = f1 ? nkb1 : nkb2;
+          const int32_t arow = (int32_t)(e * (uint32_t)p.cap_rows + t.b * 128u);
+          const uint32_t bytes = (uint32_t)kStageB + (pair ? 2u : 1u) * (uint32_t)kStageA;
+          ptx::fence_proxy_async();  // rows / activations were written with generic stores
+          bool ok = true;
+          for (uint32_t kb = 0; kb < nkb; ++kb, ++wide_it) {
+            const uint32_t s = wide_it % kWideStages, sph = (wide_it / kWideStages) & 1u;
+            ok = wait_bar_warp(p, sc, &sc.wide_empty[s], sph ^ 1u, FDMOE_ERR_TIMEOUT_STAGE);
+            if (!ok) break;
+            uint8_t* sa = stage + s * kWideBytes;
+            uint8_t* sb = sa + 2 * kStageA;
+            if (elected) {
+              uint64_t* bar = &sc.wide_full[s];
+              ptx::mbar_expect_tx(bar, bytes);
+              const int32_t kx = (int32_t)(kb * FDMOE_TILE_K);
+              const FdmoeTensorMap* ta = f1 ? &p.tm_packed : &p.tm_act;
+              ptx::tma_load_2d(sa, ta, bar, kx, arow);
+              if (pair) ptx::tma_load_2d(sa + kStageA, ta, bar, kx, arow + 128);
+              if (f1) {
+                const int32_t brow = (int32_t)(e * 2u * (uint32_t)p.I + n * FDMOE_TILE_N1);
+                ptx::tma_load_2d(sb, &p.tm_w13, bar, kx, brow);
+                ptx::tma_load_2d(sb + kStageA, &p.tm_w13, bar, kx, brow + p.I);
+              } else {
+                ptx::tma_load_2d(sb, &p.tm_w2, bar, kx, (int32_t)(e * (uint32_t)p.H + n * FDMOE_TILE_N2));
+              }
+            }
+            __syncwarp();
+          }
+          if (!ok) break;
+        } else
         if (kind == FDMOE_TASK_FFN1 || kind == FDMOE_TASK_FFN2 || kind == FDMOE_TASK_GATE) {
           const uint32_t e = (t.a >> 8) & 0xfffu, n = t.a >> 20, j = t.b;
           const bool f1 = kind == FDMOE_TASK_FFN1, gt = kind == FDMOE_TASK_GATE;
@@ -1473,7 +1561,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
       const bool elected = ptx::elect_one();
       constexpr uint32_t idesc256 = ptx::make_idesc_bf16(128, 256);
       constexpr uint32_t idesc128 = ptx::make_idesc_bf16(128, 128);
-      uint32_t stage_it = 0, tile_it = 0, skips = 0;
+      uint32_t stage_it = 0, wide_it = 0, tile_it = 0, skips = 0;
       for (uint32_t it = 0;; ++it) {
         const uint32_t r = it % kRing, ph = (it / kRing) & 1u;
         if (!wait_bar_warp(p, sc, &sc.ring_full[r], ph, FDMOE_ERR_TIMEOUT_RING, 2u)) break;
@@ -1481,7 +1569,66 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
         const uint32_t kind = t.a & 0xffu;
         if (kind == FDMOE_TASK_EXIT) break;
         bool ok = true;
-        if (kind == FDMOE_TASK_FFN1 || kind == FDMOE_TASK_FFN2 || kind == FDMOE_TASK_GATE) {
+        if ((kind == FDMOE_TASK_FFN1 || kind == FDMOE_TASK_FFN2) && (t.c & FDMOE_TILE_WIDE) != 0u) {
+          // One k-block of weights against two blocks of 128 rows, an accumulator each.  The second
+          // accumulator may still be read by the previous task's epilogue: the first one then runs
+          // ahead, as far as there are stages.
+          const uint32_t nkb = (kind == FDMOE_TASK_FFN2) ? nkb2 : nkb1;
+          const bool pair = (t.c & FDMOE_TILE_ROWS) > 128u;
+          const uint32_t acc0 = tile_it & 1u, aph0 = (tile_it >> 1) & 1u;
+          const uint32_t acc1 = acc0 ^ 1u, aph1 = ((tile_it + 1u) >> 1) & 1u;
+          tile_it += pair ? 2u : 1u;
+          if (!wait_bar_warp(p, sc, &sc.tmem_empty[acc0], aph0 ^ 1u, FDMOE_ERR_TIMEOUT_TMEM)) break;
+          ptx::tcgen05_fence_after();
+          bool ready1 = false;
+          uint32_t kb1 = 0, it1 = wide_it;  // the second accumulator's next k-block and its stage use
+          for (uint32_t kb = 0; kb < nkb; ++kb, ++wide_it) {
+            const uint32_t s = wide_it % kWideStages, sph = (wide_it / kWideStages) & 1u;
+            ok = wait_bar_warp(p, sc, &sc.wide_full[s], sph, FDMOE_ERR_TIMEOUT_STAGE);
+            if (!ok) break;
+            ptx::tcgen05_fence_after();
+            if (elected) {
+              const uint32_t sa = ptx::smem_u32(stage + s * kWideBytes);
+              const uint64_t da = ptx::make_smem_desc_sw128(sa), db = ptx::make_smem_desc_sw128(sa + 2 * kStageA);
+#pragma unroll
+              for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4)
+                ptx::umma_bf16(tmem_base + acc0 * kAccCols, da + k4 * 2u, db + k4 * 2u, idesc256, (kb | k4) != 0u);
+              if (!pair) ptx::umma_commit(&sc.wide_empty[s]);
+              if (kb == nkb - 1u) ptx::umma_commit(&sc.tmem_full[acc0]);
+            }
+            __syncwarp();
+            if (!pair) continue;
+            if (!ready1) {
+              if (kb == nkb - 1u || kb - kb1 == kWideStages - 1u) {
+                ok = wait_bar_warp(p, sc, &sc.tmem_empty[acc1], aph1 ^ 1u, FDMOE_ERR_TIMEOUT_TMEM);
+                if (!ok) break;
+                ready1 = true;
+              } else {
+                ready1 = __all_sync(0xffffffffu, ptx::mbar_test_wait(&sc.tmem_empty[acc1], aph1 ^ 1u));
+              }
+              if (ready1) ptx::tcgen05_fence_after();
+            }
+            if (ready1) {
+              if (elected) {
+                for (; kb1 <= kb; ++kb1, ++it1) {
+                  const uint32_t s1 = it1 % kWideStages;
+                  const uint32_t sa = ptx::smem_u32(stage + s1 * kWideBytes);
+                  const uint64_t da = ptx::make_smem_desc_sw128(sa + kStageA);
+                  const uint64_t db = ptx::make_smem_desc_sw128(sa + 2 * kStageA);
+#pragma unroll
+                  for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4)
+                    ptx::umma_bf16(tmem_base + acc1 * kAccCols, da + k4 * 2u, db + k4 * 2u, idesc256, (kb1 | k4) != 0u);
+                  ptx::umma_commit(&sc.wide_empty[s1]);
+                }
+                if (kb == nkb - 1u) ptx::umma_commit(&sc.tmem_full[acc1]);
+              }
+              __syncwarp();
+              it1 = wide_it + 1u;  // the same for every lane
+              kb1 = kb + 1u;
+            }
+          }
+          if (!ok) break;
+        } else if (kind == FDMOE_TASK_FFN1 || kind == FDMOE_TASK_FFN2 || kind == FDMOE_TASK_GATE) {
           const uint32_t nkb = (kind == FDMOE_TASK_FFN2) ? nkb2 : nkb1;
           const uint32_t idesc = (kind == FDMOE_TASK_GATE) ? idesc128 : idesc256;
           const uint32_t acc = tile_it & 1u, aph = (tile_it >> 1) & 1u;
@@ -1584,21 +1731,32 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           sc.skip_done = sc.skip_done + 1u;
         }
       } else if (kind == FDMOE_TASK_FFN1 || kind == FDMOE_TASK_FFN2) {
-        const uint32_t acc = tile_it & 1u, aph = (tile_it >> 1) & 1u;
-        ++tile_it;
-        stage_it += (kind == FDMOE_TASK_FFN1) ? nkb1 : nkb2;
-        if (!epi_vote_all(wait_bar(p, sc, &sc.tmem_full[acc], aph, FDMOE_ERR_TIMEOUT_TMEM))) break;
-        if (p.prof && etid == 0) pt1 = prof_now();
-        ptx::tcgen05_fence_after();
-        const uint32_t taddr = tmem_base + acc * kAccCols;
-        bool remote = false;
-        if (kind == FDMOE_TASK_FFN1)
-          ffn1_epilogue(p, sc, taddr, q, h, lane, ewarp, e, j, n, rows);
-        else
-          remote = ffn2_epilogue(p, sc, taddr, q, h, lane, ewarp, e, j, n, rows);
-        ptx::tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&sc.tmem_empty[acc]);
+        const uint32_t trows = rows & FDMOE_TILE_ROWS, halves = trows > 128u ? 2u : 1u;
+        if (!(rows & FDMOE_TILE_WIDE)) stage_it += (kind == FDMOE_TASK_FFN1) ? nkb1 : nkb2;
+        bool remote = false, landed = true;
+        for (uint32_t hf = 0; hf < halves; ++hf) {
+          const uint32_t hrows = min(128u, trows - hf * 128u);
+          const uint32_t acc = tile_it & 1u, aph = (tile_it >> 1) & 1u;
+          ++tile_it;
+          const uint32_t taddr = tmem_base + acc * kAccCols;
+          if (kind == FDMOE_TASK_FFN1) {
+            landed = epi_vote_all(wait_bar(p, sc, &sc.tmem_full[acc], aph, FDMOE_ERR_TIMEOUT_TMEM));
+            if (!landed) break;
+            if (p.prof && etid == 0 && hf == 0) pt1 = prof_now();
+            ptx::tcgen05_fence_after();
+            ffn1_epilogue(p, sc, taddr, &sc.tmem_empty[acc], q, h, lane, ewarp, e, j + hf, n, hrows);
+          } else {
+            // the row's destination comes from global memory: asked for before the accumulator is waited for
+            const YRow y = ffn2_row(p, q, h, lane, e, j + hf, n, hrows);
+            landed = epi_vote_all(wait_bar(p, sc, &sc.tmem_full[acc], aph, FDMOE_ERR_TIMEOUT_TMEM));
+            if (!landed) break;
+            if (p.prof && etid == 0 && hf == 0) pt1 = prof_now();
+            ptx::tcgen05_fence_after();
+            ffn2_epilogue(sc, taddr, &sc.tmem_empty[acc], q, h, lane, ewarp, y);
+            remote |= y.remote;
+          }
+        }
+        if (!landed) break;
         const uint32_t pta = (p.prof && etid == 0) ? prof_now() : 0u;
 
         // The tile's stores are issued.  Dependency counting, successor pushes and
@@ -1766,7 +1924,8 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           running = false;
           break;
         }
-        const uint32_t e = (t.a >> 8) & 0xfffu, j = t.b, rows = t.c;
+        // (a wide task's m-tiles are counted together, under the first one)
+        const uint32_t e = (t.a >> 8) & 0xfffu, j = t.b, rows = t.c & FDMOE_TILE_ROWS;
         if (kind == FDMOE_TASK_FFN1) {
           if (lane == 0) {
             const uint32_t prev = atomicAdd(&p.ffn1_done[(size_t)e * p.MT + j], 1u);
@@ -1776,7 +1935,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
               queue_push<false>(p, me, 0, nt2, [&](uint32_t i3, uint32_t& a, uint32_t& b, uint32_t& c) {
                 a = task_word(FDMOE_TASK_FFN2, e, i3);
                 b = j;
-                c = rows;
+                c = t.c;
               });
             }
           }
@@ -1791,86 +1950,88 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
             // to four rows; it first counts them all, then publishes the groups it completed with one
             // fence for the whole warp (the last m-tiles of a launch complete dozens of groups each).
             fence_acqrel<false>();
-            uint32_t c_home[4], c_first[4], c_ntok[4], nc = 0u;
-            // (the four counter updates of a lane are issued back to back, their results are looked
-            // at afterwards: over NVLink each takes microseconds to answer)
-            uint32_t r_home[4], r_first[4], r_ntok[4], r_got[4];
-#pragma unroll
-            for (uint32_t rr = 0; rr < 4u; ++rr) {
-              const uint32_t r = rr * 32u + (uint32_t)lane;
-              r_home[rr] = 0xffffffffu;
-              r_first[rr] = 0u;
-              r_ntok[rr] = 0u;
-              r_got[rr] = 0u;
-              c_home[rr] = 0u;
-              c_first[rr] = 0u;
-              c_ntok[rr] = 0u;
-              if (r < rows) {
-                const uint4 mraw = ld_cg_u4(&me.meta[(size_t)e * p.cap_rows + (size_t)j * 128 + r]);
-                const int hm = (int)mraw.y >> 8;
-                const uint32_t g = mraw.x / G;
-                const uint32_t th = tokens_of_rank(p, hm);
-                r_home[rr] = (uint32_t)hm;
-                r_first[rr] = g * G;
-                r_ntok[rr] = min(G, th - g * G);
-                if (S && hm != p.rank)
-                  r_got[rr] = atom_add<true>(&p.peers[hm].grp_cnt[g], 1u) + 1u;
-                else
-                  r_got[rr] = atom_add<false>(&p.peers[hm].grp_cnt[g], 1u) + 1u;
-              }
-            }
-#pragma unroll
-            for (uint32_t rr = 0; rr < 4u; ++rr) {
-              if (r_home[rr] != 0xffffffffu && r_got[rr] == r_ntok[rr] * (uint32_t)p.K) {
-#pragma unroll
-                for (uint32_t c = 0; c < 4u; ++c) {
-                  if (c == nc) {
-                    c_home[c] = r_home[rr];
-                    c_first[c] = r_first[rr];
-                    c_ntok[c] = r_ntok[rr];
-                  }
+            for (uint32_t row0 = 0; row0 < rows; row0 += 128u) {
+              uint32_t c_home[4], c_first[4], c_ntok[4], nc = 0u;
+              // (the four counter updates of a lane are issued back to back, their results are looked
+              // at afterwards: over NVLink each takes microseconds to answer)
+              uint32_t r_home[4], r_first[4], r_ntok[4], r_got[4];
+  #pragma unroll
+              for (uint32_t rr = 0; rr < 4u; ++rr) {
+                const uint32_t r = row0 + rr * 32u + (uint32_t)lane;
+                r_home[rr] = 0xffffffffu;
+                r_first[rr] = 0u;
+                r_ntok[rr] = 0u;
+                r_got[rr] = 0u;
+                c_home[rr] = 0u;
+                c_first[rr] = 0u;
+                c_ntok[rr] = 0u;
+                if (r < rows) {
+                  const uint4 mraw = ld_cg_u4(&me.meta[(size_t)e * p.cap_rows + (size_t)j * 128 + r]);
+                  const int hm = (int)mraw.y >> 8;
+                  const uint32_t g = mraw.x / G;
+                  const uint32_t th = tokens_of_rank(p, hm);
+                  r_home[rr] = (uint32_t)hm;
+                  r_first[rr] = g * G;
+                  r_ntok[rr] = min(G, th - g * G);
+                  if (S && hm != p.rank)
+                    r_got[rr] = atom_add<true>(&p.peers[hm].grp_cnt[g], 1u) + 1u;
+                  else
+                    r_got[rr] = atom_add<false>(&p.peers[hm].grp_cnt[g], 1u) + 1u;
                 }
-                ++nc;
               }
-            }
-            uint32_t ticket[4];
-            bool any_remote = false;
-#pragma unroll
-            for (uint32_t c = 0; c < 4u; ++c) {
-              ticket[c] = 0u;
-              if (c < nc) {
-                const FdmoePeer& hp = p.peers[c_home[c]];
-                const bool rem = S && (int)c_home[c] != p.rank;
-                any_remote |= rem;
-                ticket[c] = rem ? atom_add<true>(&hp.ctl->q[0].head, 1u) : atom_add<false>(&hp.ctl->q[0].head, 1u);
-                FdmoeSlot* sl = &hp.slots[0][ticket[c] & (uint32_t)p.queue_mask];
-                sl->a = FDMOE_TASK_COMBINE;
-                sl->b = c_first[c];
-                sl->c = c_ntok[c];
+  #pragma unroll
+              for (uint32_t rr = 0; rr < 4u; ++rr) {
+                if (r_home[rr] != 0xffffffffu && r_got[rr] == r_ntok[rr] * (uint32_t)p.K) {
+  #pragma unroll
+                  for (uint32_t c = 0; c < 4u; ++c) {
+                    if (c == nc) {
+                      c_home[c] = r_home[rr];
+                      c_first[c] = r_first[rr];
+                      c_ntok[c] = r_ntok[rr];
+                    }
+                  }
+                  ++nc;
+                }
               }
-            }
-            if (__any_sync(0xffffffffu, nc != 0u)) {
-              if (__any_sync(0xffffffffu, any_remote))
-                fence_acqrel<true>();
-              else
-                fence_acqrel<false>();
-#pragma unroll
+              uint32_t ticket[4];
+              bool any_remote = false;
+  #pragma unroll
               for (uint32_t c = 0; c < 4u; ++c) {
+                ticket[c] = 0u;
                 if (c < nc) {
                   const FdmoePeer& hp = p.peers[c_home[c]];
-                  if (S && (int)c_home[c] != p.rank) {
-                    st_relaxed<true>(&hp.slots[0][ticket[c] & (uint32_t)p.queue_mask].seq, ticket[c] + 1u);
-                    atom_add<true>(&hp.ctl->q[0].avail, 1u);
-                  } else {
-                    st_relaxed<false>(&hp.slots[0][ticket[c] & (uint32_t)p.queue_mask].seq, ticket[c] + 1u);
-                    atom_add<false>(&hp.ctl->q[0].avail, 1u);
+                  const bool rem = S && (int)c_home[c] != p.rank;
+                  any_remote |= rem;
+                  ticket[c] = rem ? atom_add<true>(&hp.ctl->q[0].head, 1u) : atom_add<false>(&hp.ctl->q[0].head, 1u);
+                  FdmoeSlot* sl = &hp.slots[0][ticket[c] & (uint32_t)p.queue_mask];
+                  sl->a = FDMOE_TASK_COMBINE;
+                  sl->b = c_first[c];
+                  sl->c = c_ntok[c];
+                }
+              }
+              if (__any_sync(0xffffffffu, nc != 0u)) {
+                if (__any_sync(0xffffffffu, any_remote))
+                  fence_acqrel<true>();
+                else
+                  fence_acqrel<false>();
+  #pragma unroll
+                for (uint32_t c = 0; c < 4u; ++c) {
+                  if (c < nc) {
+                    const FdmoePeer& hp = p.peers[c_home[c]];
+                    if (S && (int)c_home[c] != p.rank) {
+                      st_relaxed<true>(&hp.slots[0][ticket[c] & (uint32_t)p.queue_mask].seq, ticket[c] + 1u);
+                      atom_add<true>(&hp.ctl->q[0].avail, 1u);
+                    } else {
+                      st_relaxed<false>(&hp.slots[0][ticket[c] & (uint32_t)p.queue_mask].seq, ticket[c] + 1u);
+                      atom_add<false>(&hp.ctl->q[0].avail, 1u);
+                    }
                   }
                 }
               }
             }
             __syncwarp();
             if (lane == 0) {
-              atomicAdd(&ctl->mtiles_done, 1u);
+              atomicAdd(&ctl->mtiles_done, (rows + 127u) / 128u);
               maybe_close(p);
             }
           }

@@ -51,13 +51,26 @@ enum {
   FDMOE_ERR_ROW_OVERFLOW = 8,    // more rows for an expert than its buffer holds
 };
 
+// The third word of an FFN1 / FFN2 task: valid rows of the tile (up to 128; a wide one's up to 256) and
+// whether it is wide.  A wide task runs two m-tiles of an expert against each block of weights, which
+// brings 64 KB of operands into shared memory for what costs two narrow ones 96 KB.  On one GPU an
+// expert's tasks are wide from 129 rows on: below there is no second m-tile, and from there on both
+// forms were measured (B200, whole layer, narrow and wide): 16384 tokens of the 2048 x 768 shape
+// 1560 and 1513 us, 4096 tokens 551 and 552 us, 2048 tokens of the 4096 x 1536 shape 1226 and 1161 us.
+// With peers they stay narrow: a wide task holds both accumulators through its epilogue, whose stores
+// cross NVLink there.
+enum {
+  FDMOE_TILE_ROWS = 0xffff,
+  FDMOE_TILE_WIDE = 1 << 16,
+};
+
 // One slot of a task queue (16 bytes).  `seq` == ticket + 1 once the slot
 // holds the task of that ticket.
 typedef struct {
   uint32_t seq;
   uint32_t a;  // kind | expert << 8 | n_tile << 20
   uint32_t b;  // m_tile, or first token, or chunk index
-  uint32_t c;  // valid rows in the tile, or token count
+  uint32_t c;  // valid rows in the tile (and FDMOE_TILE_WIDE), or token count
 } FdmoeSlot;
 
 // Sideband of one packed row (16 bytes): where its result goes.

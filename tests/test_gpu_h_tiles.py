@@ -1,0 +1,27 @@
+"""GPU parity at the edges of the FFN tiles: every token selects the same experts, so that each of them
+holds exactly as many (different) rows as there are tokens, and all others none."""
+import pytest
+
+import moe_testlib as tl
+from moe_testlib import synth
+from test_gpu_b_stages import check_layer
+
+pytestmark = pytest.mark.gpu
+
+
+def same_experts(tokens):
+    s = synth.TINY
+    gate, w13, w2 = synth.make_weights(s, seed=7, std=0.05)
+    x = synth.make_tokens(s, tokens, seed=7)
+    x[:, -1] = 1.0
+    gate[:, -1] = 0.0
+    gate[[3, 11, 18, 30], -1] = tl.torch.tensor([40.0, 36.0, 32.0, 28.0], dtype=gate.dtype)
+    return s, x, gate, w13, w2
+
+
+# one m-tile and two; a wide task's second half with one row, part of a box of rows, and full; a wide task
+# of one m-tile behind a full one
+@pytest.mark.parametrize("rows", [128, 129, 200, 255, 256, 257, 384, 385])
+def test_rows_per_expert_at_the_edges_of_wide_tiles(rows):
+    s, x, gate, w13, w2 = same_experts(rows)
+    check_layer(s, x, gate, w13, w2, max_tokens=rows)
