@@ -295,6 +295,8 @@ cudaError_t MoeKernelLauncher::Init(const void* gateW, const void* w13, const vo
   }
   const uint64_t exp_rows = (uint64_t)g_.El * g_.cap_rows;
   CUDA_ERROR_CHECK(MakeTensorMap(enc, &params_.tm_packed, arena_ + layout_.packed, exp_rows, g_.H, 128));
+  CUDA_ERROR_CHECK(MakeTensorMap(enc, &params_.tm_packed_box, arena_ + layout_.packed, exp_rows, g_.H, FDMOE_ROW_BOX));
+  CUDA_ERROR_CHECK(MakeTensorMap(enc, &params_.tm_act_box, act_, exp_rows, g_.I, FDMOE_ROW_BOX));
   CUDA_ERROR_CHECK(MakeTensorMap(enc, &params_.tm_w13, w13_dev, (uint64_t)g_.El * 2 * g_.I, g_.H, 128));
   CUDA_ERROR_CHECK(MakeTensorMap(enc, &params_.tm_act, act_, exp_rows, g_.I, 128));
   CUDA_ERROR_CHECK(MakeTensorMap(enc, &params_.tm_w2, w2_dev, (uint64_t)g_.El * g_.H, g_.I, 256));

@@ -1238,6 +1238,24 @@ __device__ __forceinline__ uint32_t gate_kblocks_per_stage(bool is_gate, int gat
   return (is_gate && gate_rows <= 64) ? 2u : 1u;
 }
 
+// Brings `rows` (1..128) rows of an expert's buffer, one k-block wide, into a stage: in boxes of 16 rows
+// up to 64, else in one box of 128.  The stage's other rows keep what was there: they only reach
+// accumulator rows that nobody reads.  In a decode batch an expert holds a handful of rows, and a box of
+// 128 is a third of all operand bytes, most of it from DRAM since nothing ever wrote it.  Whole layer at 128
+// tokens of the 2048 x 768 shape: 294 us with boxes of 128, 288 us so; at 333 tokens 300 and 296 us.
+__device__ __forceinline__ uint32_t row_load_bytes(uint32_t rows) {
+  return rows > 64u ? (uint32_t)kStageA : ((rows + 15u) / 16u) * (uint32_t)(FDMOE_ROW_BOX * FDMOE_TILE_K * 2);
+}
+__device__ __forceinline__ void load_rows(uint8_t* dst, const FdmoeTensorMap* full, const FdmoeTensorMap* box,
+                                          uint64_t* bar, int32_t kx, int32_t row0, uint32_t rows) {
+  if (rows > 64u) {
+    ptx::tma_load_2d(dst, full, bar, kx, row0);
+  } else {
+    for (uint32_t r = 0; r < rows; r += FDMOE_ROW_BOX)
+      ptx::tma_load_2d(dst + r * (FDMOE_TILE_K * 2), box, bar, kx, row0 + (int32_t)r);
+  }
+}
+
 // Pipeline stages a DISPATCH task of `nt` tokens takes (whole token rows per stage).
 __device__ __forceinline__ uint32_t dispatch_stages(const FdmoeParams& p, uint32_t nt) {
   const uint32_t rps = dispatch_rows_per_stage(p.H);
@@ -1317,6 +1335,8 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
     ptx::prefetch_tmap(&p.tm_packed);
     ptx::prefetch_tmap(&p.tm_w13);
     ptx::prefetch_tmap(&p.tm_act);
+    ptx::prefetch_tmap(&p.tm_packed_box);
+    ptx::prefetch_tmap(&p.tm_act_box);
     ptx::prefetch_tmap(&p.tm_w2);
     ptx::prefetch_tmap(&p.tm_x);
     ptx::prefetch_tmap(&p.tm_gate);
@@ -1421,7 +1441,8 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           const bool f1 = kind == FDMOE_TASK_FFN1, pair = rows > 128u;
           const uint32_t nkb = f1 ? nkb1 : nkb2;
           const int32_t arow = (int32_t)(e * (uint32_t)p.cap_rows + t.b * 128u);
-          const uint32_t bytes = (uint32_t)kStageB + (pair ? 2u : 1u) * (uint32_t)kStageA;
+          const uint32_t bytes =
+              (uint32_t)kStageB + (pair ? (uint32_t)kStageA + row_load_bytes(rows - 128u) : row_load_bytes(rows));
           ptx::fence_proxy_async();  // rows / activations were written with generic stores
           bool ok = true;
           for (uint32_t kb = 0; kb < nkb; ++kb, ++wide_it) {
@@ -1434,9 +1455,9 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
               uint64_t* bar = &sc.wide_full[s];
               ptx::mbar_expect_tx(bar, bytes);
               const int32_t kx = (int32_t)(kb * FDMOE_TILE_K);
-              const FdmoeTensorMap* ta = f1 ? &p.tm_packed : &p.tm_act;
-              ptx::tma_load_2d(sa, ta, bar, kx, arow);
-              if (pair) ptx::tma_load_2d(sa + kStageA, ta, bar, kx, arow + 128);
+              const FdmoeTensorMap *ta = f1 ? &p.tm_packed : &p.tm_act, *tb = f1 ? &p.tm_packed_box : &p.tm_act_box;
+              load_rows(sa, ta, tb, bar, kx, arow, min(rows, 128u));
+              if (pair) load_rows(sa + kStageA, ta, tb, bar, kx, arow + 128, rows - 128u);
               if (f1) {
                 const int32_t brow = (int32_t)(e * 2u * (uint32_t)p.I + n * FDMOE_TILE_N1);
                 ptx::tma_load_2d(sb, &p.tm_w13, bar, kx, brow);
@@ -1459,6 +1480,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           // GATE tiles of up to 64 tokens are bound by the round trip of a stage, not by its size:
           // they put two k-blocks into one stage (A 2 x 8 KB, B 2 x 16 KB)
           const uint32_t gk = gate_kblocks_per_stage(gt, p.gate_rows);
+          const uint32_t bytes = gt ? gk * gate_bytes : (uint32_t)kStageB + row_load_bytes(t.c);
           ptx::fence_proxy_async();  // rows / activations were written with generic stores
           bool ok = true;
           for (uint32_t kb = 0; kb < nkb && ok; kb += gk, ++stage_it) {
@@ -1468,7 +1490,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
             uint8_t* sa = stage + s * kStageBytes;
             uint8_t* sb = sa + kStageA;
             if (elected) {
-              ptx::mbar_expect_tx(&sc.full_bar[s], gt ? gk * gate_bytes : (uint32_t)kStageBytes);
+              ptx::mbar_expect_tx(&sc.full_bar[s], bytes);
               const int32_t kx = (int32_t)(kb * FDMOE_TILE_K);
               if (gt) {
                 for (uint32_t i = 0; i < gk; ++i) {
@@ -1476,12 +1498,12 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
                   ptx::tma_load_2d(sb + i * kStageA, &p.tm_gate, &sc.full_bar[s], kx + (int32_t)(i * FDMOE_TILE_K), 0);
                 }
               } else if (f1) {
-                ptx::tma_load_2d(sa, &p.tm_packed, &sc.full_bar[s], kx, arow);
+                load_rows(sa, &p.tm_packed, &p.tm_packed_box, &sc.full_bar[s], kx, arow, t.c);
                 const int32_t brow = (int32_t)(e * 2u * (uint32_t)p.I + n * FDMOE_TILE_N1);
                 ptx::tma_load_2d(sb, &p.tm_w13, &sc.full_bar[s], kx, brow);
                 ptx::tma_load_2d(sb + kStageA, &p.tm_w13, &sc.full_bar[s], kx, brow + p.I);
               } else {
-                ptx::tma_load_2d(sa, &p.tm_act, &sc.full_bar[s], kx, arow);
+                load_rows(sa, &p.tm_act, &p.tm_act_box, &sc.full_bar[s], kx, arow, t.c);
                 const int32_t brow = (int32_t)(e * (uint32_t)p.H + n * FDMOE_TILE_N2);
                 ptx::tma_load_2d(sb, &p.tm_w2, &sc.full_bar[s], kx, brow);
               }

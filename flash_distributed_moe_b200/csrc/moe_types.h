@@ -16,6 +16,7 @@ enum {
   FDMOE_TILE_N1 = 128,   // FFN1: activation columns per tile (MMA N = 2 * 128: gate + up)
   FDMOE_TILE_N2 = 256,   // FFN2: hidden columns per tile
   FDMOE_TILE_K = 64,     // one 128-byte swizzle atom of bf16 per stage
+  FDMOE_ROW_BOX = 16,      // rows per load of an FFN tile with few rows
   FDMOE_GATE_TOKENS = 128,  // tokens per gate tile (one tcgen05 M tile)
 };
 
@@ -140,6 +141,8 @@ typedef struct __attribute__((aligned(64))) {
 
 typedef struct {
   FdmoeTensorMap tm_packed;  // [El*cap_rows, H]   box 64 x 128
+  FdmoeTensorMap tm_packed_box;  // the same, box 64 x 16
+  FdmoeTensorMap tm_act_box;     // [El*cap_rows, I]   box 64 x 16
   FdmoeTensorMap tm_w13;     // [El*2I, H]         box 64 x 128
   FdmoeTensorMap tm_act;     // [El*cap_rows, I]   box 64 x 128
   FdmoeTensorMap tm_w2;      // [El*H, I]          box 64 x 256

@@ -162,6 +162,8 @@ extern "C" int FlashMoeLaunchNoAlloc(const void* gateWeights, const void* ffn1Ex
   memset(&p, 0, sizeof(p));
   const uint64_t exp_rows = (uint64_t)g.El * g.cap_rows;
   NA_CHECK(MakeTensorMap(d->encode, &p.tm_packed, base + L.packed, exp_rows, g.H, 128));
+  NA_CHECK(MakeTensorMap(d->encode, &p.tm_packed_box, base + L.packed, exp_rows, g.H, FDMOE_ROW_BOX));
+  NA_CHECK(MakeTensorMap(d->encode, &p.tm_act_box, base + off_act, exp_rows, g.I, FDMOE_ROW_BOX));
   NA_CHECK(MakeTensorMap(d->encode, &p.tm_w13, ffn1ExpertWeights, (uint64_t)g.El * 2 * g.I, g.H, 128));
   NA_CHECK(MakeTensorMap(d->encode, &p.tm_act, base + off_act, exp_rows, g.I, 128));
   NA_CHECK(MakeTensorMap(d->encode, &p.tm_w2, ffn2ExpertWeights, (uint64_t)g.El * g.H, g.I, 256));

@@ -25,3 +25,10 @@ def same_experts(tokens):
 def test_rows_per_expert_at_the_edges_of_wide_tiles(rows):
     s, x, gate, w13, w2 = same_experts(rows)
     check_layer(s, x, gate, w13, w2, max_tokens=rows)
+
+
+# the edges of the 16-row boxes that tiles of up to 64 rows are loaded in
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 33, 48, 64, 65, 127])
+def test_rows_per_expert_at_the_edges_of_row_boxes(rows):
+    s, x, gate, w13, w2 = same_experts(rows)
+    check_layer(s, x, gate, w13, w2, max_tokens=128)
