@@ -395,15 +395,15 @@ cudaError_t MoeKernelLauncher::LaunchBf16(const void* tokens, void* output, int 
   FdmoeParams p = params_;
   if (tokensNum > 0 && mode == 0) {
     // the token matrix moves between launches: its TMA descriptor is rebuilt (host-only arithmetic)
-    // GATE tile height: the smallest of 32/64/128 tokens that still gives every SM at most one tile,
-    // so that the gate phase spreads over as many SMs as possible
-    // (with peers: always 32, many small tiles let the tensor cores start on the first rows while
-    // later tiles are still being dispatched over NVLink)
-    int rows = 128;
-    if (tokensNum <= 32 * grid_ || world_ > 1) rows = 32;
-    else if (tokensNum <= 64 * grid_) rows = 64;
+    // (with peers: always GATE tiles of 32 tokens, many small tiles let the tensor cores start on the
+    // first rows while later tiles are still being dispatched over NVLink; the dump of the tensor-core
+    // logits needs GATE tiles too)
+    int rows = GateRows(tokensNum, grid_);
+    if (world_ > 1 || (debug_logits_ && rows < 32)) rows = 32;
     p.gate_rows = EnvInt("FLASHMOE_GATE_ROWS", rows);
-    if (p.gate_rows != 32 && p.gate_rows != 64 && p.gate_rows != 128) p.gate_rows = rows;
+    const bool exact = p.gate_rows == 1 || p.gate_rows == 2;
+    if (exact ? world_ > 1 || debug_logits_ : p.gate_rows != 32 && p.gate_rows != 64 && p.gate_rows != 128)
+      p.gate_rows = rows;
     CUDA_ERROR_CHECK(MakeTensorMap(encode_, &p.tm_x, tokens, (uint64_t)tokensNum, g_.H,
                                    std::min(p.gate_rows, tokensNum)));
   }

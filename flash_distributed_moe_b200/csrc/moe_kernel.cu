@@ -106,10 +106,14 @@ struct __align__(64) SmemCtl {
       uint8_t lpos[FDMOE_GATE_TOKENS][FDMOE_MAX_TOPK];
     };
     struct {
-      // GATEFIX task scratch: two token rows and their exact logits
-      uint4 xrow[2][FDMOE_MAX_HIDDEN / 8];
-      float exact[2][128];
-      uint2 fix_dst[2][FDMOE_MAX_TOPK];         // {expert, row in the owner's buffers} of each slot, or {~0, 0}
+      // GATEFIX task scratch: two token rows as fp32, later their exact logits and destinations
+      union {
+        float xrow[2][FDMOE_MAX_HIDDEN];
+        struct {
+          float exact[2][128];
+          uint2 fix_dst[2][FDMOE_MAX_TOPK];     // {expert, row in the owner's buffers} of each slot, or {~0, 0}
+        };
+      };
     };
     // FFN epilogues: per-warp staging of 32 rows x 128 bytes (chunks swizzled within a row)
     uint8_t store_stage[kEpiThreads / 32][32 * 128];
@@ -439,9 +443,17 @@ __device__ __forceinline__ FdmoeSlot next_task(const FdmoeParams& p, SmemCtl& sc
       const uint32_t g = atomicAdd(&ctl->gate_next, 1u);
       if (g < gate_tiles) {
         out.seq = 0;
-        out.a = FDMOE_TASK_GATE;
-        out.b = g;
-        out.c = 0;
+        if (p.gate_rows <= 2) {
+          // few tokens: gated exactly, one or two per task (GateRows draws the line)
+          const uint32_t t = g * (uint32_t)p.gate_rows;
+          out.a = FDMOE_TASK_GATEFIX;
+          out.b = t;
+          out.c = (p.gate_rows == 2 && t + 1u < (uint32_t)p.T) ? t + 1u : 0xffffffffu;
+        } else {
+          out.a = FDMOE_TASK_GATE;
+          out.b = g;
+          out.c = 0;
+        }
         return out;
       }
     }
@@ -474,12 +486,12 @@ __device__ __forceinline__ void maybe_close(const FdmoeParams& p) {
 // that completes a batch of an expert publishes its FFN1 tiles at once, so the tensor cores
 // start while rows are still travelling; every batch of an expert re-reads the expert's weights,
 // which is cheap when a rank holds few experts (their weights stay in L2) and expensive when it
-// holds all of them.  One GPU: no batches, every expert is published whole once gating has
-// finished.  More GPUs: about `world` batches per expert, at least two m-tiles each.
+// holds all of them.  One GPU: no batches (more m-tiles than a buffer holds: landed rows are not even
+// counted), every expert is published whole once gating has finished.  More GPUs: about `world` batches per expert, at least two m-tiles each.
 // A pure function of values every rank knows, so that all ranks agree.
 __device__ __forceinline__ uint32_t batch_mt_of(const FdmoeParams& p, uint32_t tokens_all) {
   if (p.batch_mt > 0) return (uint32_t)min(p.batch_mt, p.MT);
-  if (p.world == 1) return (uint32_t)p.MT;
+  if (p.world == 1) return (uint32_t)p.MT + 1u;
   const uint32_t mt_expert = (uint32_t)(((uint64_t)tokens_all * p.K / p.E) / FDMOE_TILE_M);
   const uint32_t b = mt_expert / (uint32_t)p.world;
   if (b < 2u) return (uint32_t)p.MT;
@@ -567,16 +579,17 @@ __device__ __forceinline__ float key_to_float(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// Warp-wide top-k of four rows of 128 logits at once (lane l owns experts l,
+// Warp-wide top-k of R rows of 128 logits at once (lane l owns experts l,
 // l+32, l+64, l+96 of each row), descending, the lower index winning ties
 // (reference refTopk.h:36-58).  Each round is one warp-wide max over the value
 // keys and one warp-wide min over the indices that hold that value
-// (redux.sync), for four independent rows.  Lane k < K ends up holding slot k.
-__device__ __forceinline__ void topk_warp4(const float* r0, int pitch, int E, int K, int lane, float (&myv)[4],
-                                           int (&myi)[4]) {
-  uint32_t key[4][4];  // key 0 marks "taken / not an expert" (no finite float maps to it)
+// (redux.sync), for R independent rows.  Lane k < K ends up holding slot k.
+template <int R>
+__device__ __forceinline__ void topk_warp(const float* r0, int pitch, int E, int K, int lane, float (&myv)[R],
+                                          int (&myi)[R]) {
+  uint32_t key[R][4];  // key 0 marks "taken / not an expert" (no finite float maps to it)
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
+  for (int r = 0; r < R; ++r) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int e = lane + 32 * i;
@@ -587,7 +600,7 @@ __device__ __forceinline__ void topk_warp4(const float* r0, int pitch, int E, in
   }
   for (int k = 0; k < K; ++k) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < R; ++r) {
       // local best: ascending i is ascending expert index, strict '>' keeps the lower one
       uint32_t bk = key[r][0];
       int bi = 0;
@@ -610,48 +623,6 @@ __device__ __forceinline__ void topk_warp4(const float* r0, int pitch, int E, in
         myv[r] = key_to_float(m);
         myi[r] = (int)win;
       }
-    }
-  }
-}
-
-// Warp-wide top-k over 128 logits in shared memory (lane l owns experts l,
-// l+32, l+64, l+96), descending, the lower index winning ties (reference
-// refTopk.h:36-58).  Result: lane k < K holds slot k.
-__device__ __forceinline__ void topk_warp(const float* logits, int E, int K, int lane, float& myv, int& myi) {
-  float v[4];
-  uint32_t taken = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int e = lane + 32 * i;
-    v[i] = (e < E) ? logits[e] : -INFINITY;
-    if (e >= E) taken |= 1u << i;
-  }
-  myv = 0.f;
-  myi = 0;
-  for (int k = 0; k < K; ++k) {
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int e = lane + 32 * i;
-      if (!((taken >> i) & 1u) && (v[i] > bv || (v[i] == bv && e < bi))) {
-        bv = v[i];
-        bi = e;
-      }
-    }
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-      if (ov > bv || (ov == bv && oi < bi)) {
-        bv = ov;
-        bi = oi;
-      }
-    }
-    if ((bi & 31) == lane && bi < 128) taken |= 1u << (bi >> 5);
-    if (lane == k) {
-      myv = bv;
-      myi = bi;
     }
   }
 }
@@ -716,7 +687,7 @@ __device__ __noinline__ void gate_epilogue(const FdmoeParams& p, SmemCtl& sc, ui
     {
       float myv[4];
       int myi[4];
-      topk_warp4(sc.logit_tile[ewarp * 4], 132, E, kk, lane, myv, myi);
+      topk_warp<4>(sc.logit_tile[ewarp * 4], 132, E, kk, lane, myv, myi);
       if (lane < kk) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -892,7 +863,7 @@ __device__ __noinline__ bool dispatch_task(const FdmoeParams& p, SmemCtl& sc, ui
   // the FFN1 tiles of every batch this completes.  One fence per signalling thread orders the rows
   // and sidebands (written by other threads of the group, before the barrier) first; it is the only
   // system-scope fence of the task, issued when nothing else of this worker is in flight.
-  if (etid < p.E && !sc.abort) {
+  if (etid < p.E && !sc.abort && sc.batch_mt <= (uint32_t)p.MT) {
     const uint32_t cnt = sc.cnt[etid];
     if (cnt) {
       const int owner = etid / p.El, le = etid - owner * p.El;
@@ -915,64 +886,97 @@ __device__ __noinline__ bool dispatch_task(const FdmoeParams& p, SmemCtl& sc, ui
 }
 
 // ================================================================== GATEFIX
-// Up to two tokens whose leading tensor-core logits were nearly tied: all E
-// logits are recomputed with fp32 FMAs in the reference's order (128 threads per
-// token, one expert each), then top-k, softmax, row reservation and the dispatch
-// of the token's K rows, i.e. everything GATE does for the other tokens.
+// The logits of one stage's columns for this thread's expert `e`: fp32 FMAs with k strictly ascending per
+// output (bf16 x bf16 products are exact in fp32, so this equals the reference's `acc += a*b` bit for bit;
+// reference refGemm.h:16-27).  The stage holds up to three 64-column boxes of gate weights (TMA, 128-byte
+// swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7)); the token rows are fp32 and broadcast.
+// A dependent FMA every four cycles is the floor of this loop.  What could hold it up is unpacking (half
+// the FMA rate) and shared-memory reads, so the token rows are unpacked once per task and one thread
+// serves both tokens, which read and unpack a weight once.
+template <bool Two>
+__device__ __forceinline__ void exact_logits(const uint8_t* stage, const float* xa, const float* xb, uint32_t e,
+                                             uint32_t blocks, float& acc_a, float& acc_b) {
+  for (uint32_t i = 0; i < blocks; ++i) {
+    const uint4* tile = reinterpret_cast<const uint4*>(stage + i * kStageA);
+    const float4* va = reinterpret_cast<const float4*>(xa + i * FDMOE_TILE_K);
+    const float4* vb = reinterpret_cast<const float4*>(xb + i * FDMOE_TILE_K);
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c) {
+      const uint4 wv = tile[e * 8 + (c ^ (e & 7))];
+      const float w[8] = {bf16_lo(wv.x), bf16_hi(wv.x), bf16_lo(wv.y), bf16_hi(wv.y),
+                          bf16_lo(wv.z), bf16_hi(wv.z), bf16_lo(wv.w), bf16_hi(wv.w)};
+#pragma unroll
+      for (uint32_t j = 0; j < 2; ++j) {
+        const float4 x = va[c * 2 + j];
+        acc_a = fmaf(x.x, w[4 * j], acc_a);
+        acc_a = fmaf(x.y, w[4 * j + 1], acc_a);
+        acc_a = fmaf(x.z, w[4 * j + 2], acc_a);
+        acc_a = fmaf(x.w, w[4 * j + 3], acc_a);
+        if (Two) {
+          const float4 y = vb[c * 2 + j];
+          acc_b = fmaf(y.x, w[4 * j], acc_b);
+          acc_b = fmaf(y.y, w[4 * j + 1], acc_b);
+          acc_b = fmaf(y.z, w[4 * j + 2], acc_b);
+          acc_b = fmaf(y.w, w[4 * j + 3], acc_b);
+        }
+      }
+    }
+  }
+}
+
+// Up to two tokens gated exactly: all E logits with fp32 FMAs in the reference's order, then top-k,
+// softmax, row reservation and the dispatch of the tokens' K rows, i.e. everything GATE and DISPATCH do
+// for the other tokens.  Published by GATE for tokens whose leading tensor-core logits were nearly tied;
+// in launches with few tokens claimed from the gate counter instead of GATE tiles.
 template <bool S>
 __device__ __noinline__ bool gatefix_task(const FdmoeParams& p, SmemCtl& sc, uint8_t* stage, uint32_t& stage_it,
                                           int etid, int ewarp, int lane, uint32_t tok_a, uint32_t tok_b) {
   const int H = p.H, E = p.E, K = p.K;
   const int half = etid >> 7, e = etid & 127;
   const uint32_t tok = half ? tok_b : tok_a;
-  const bool live = tok != 0xffffffffu;
-  const bf16* x = reinterpret_cast<const bf16*>(p.x);
+  const bool two = tok_b != 0xffffffffu, live = half == 0 || two;
+  const uint4* xsrc = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.x) + (size_t)(live ? tok : 0u) * H);
   if (live) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)tok * H);
-    for (int v = e; v < H / 8; v += 128) sc.xrow[half][v] = src[v];
+    float4* dst = reinterpret_cast<float4*>(sc.xrow[half]);
+    for (int v = e; v < H / 8; v += 128) {
+      const uint4 r = xsrc[v];
+      dst[2 * v] = make_float4(bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y));
+      dst[2 * v + 1] = make_float4(bf16_lo(r.z), bf16_hi(r.z), bf16_lo(r.w), bf16_hi(r.w));
+    }
   }
   epi_bar();
   prof_mark(p, sc, etid, 30);
-  // Exact logits: fp32 FMAs with k strictly ascending per output (bf16 x bf16
-  // products are exact in fp32, so this equals the reference's `acc += a*b` bit
-  // for bit; reference refGemm.h:16-27).  The gate weights arrive up to 192 columns
-  // (three 64-column boxes) per stage through the stage ring (TMA, 128-byte swizzle: 16-byte chunk c of row r
-  // sits at chunk c ^ (r & 7)); the token row is broadcast from shared memory.
   {
-    float acc = 0.f;
+    float acc_a = 0.f, acc_b = 0.f;
     const uint32_t nkb = (uint32_t)(H / FDMOE_TILE_K);
     for (uint32_t kb = 0; kb < nkb; kb += kFixBlocks, ++stage_it) {
       const uint32_t s = stage_it % kStages, sph = (stage_it / kStages) & 1u;
       if (!epi_vote_all(wait_bar(p, sc, &sc.full_bar[s], sph, FDMOE_ERR_TIMEOUT_STAGE))) return false;
-      if (live && e < E) {
+      if (etid < E) {  // (E <= 128: the first four warps)
         const uint32_t nb = min((uint32_t)kFixBlocks, nkb - kb);
-        for (uint32_t i = 0; i < nb; ++i) {
-          const uint4* tile = reinterpret_cast<const uint4*>(stage + s * kStageBytes + i * kStageA);
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const uint4 wv = tile[e * 8 + (c ^ (e & 7))];
-            const uint4 xv = sc.xrow[half][(kb + i) * 8 + c];
-            const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
-            const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              acc = fmaf(bf16_lo(xw[j]), bf16_lo(ww[j]), acc);
-              acc = fmaf(bf16_hi(xw[j]), bf16_hi(ww[j]), acc);
-            }
-          }
-        }
+        const uint8_t* st = stage + s * kStageBytes;
+        const float *xa = sc.xrow[0] + kb * FDMOE_TILE_K, *xb = sc.xrow[1] + kb * FDMOE_TILE_K;
+        if (two)
+          exact_logits<true>(st, xa, xb, (uint32_t)e, nb, acc_a, acc_b);
+        else
+          exact_logits<false>(st, xa, xb, (uint32_t)e, nb, acc_a, acc_b);
       }
-      epi_bar();  // every thread has read the stage
+      epi_bar();  // every thread has read the stage (and, at the end, the token rows)
       if (etid == 0) ptx::mbar_arrive(&sc.empty_bar[s]);
     }
-    if (live && e < E) sc.exact[half][e] = acc;
+    if (etid < E) {
+      sc.exact[0][e] = acc_a;
+      sc.exact[1][e] = acc_b;
+    }
   }
   epi_bar();
   prof_mark(p, sc, etid, 31);
   if (live && (ewarp & 3) == 0) {
-    float myv;
-    int myi;
-    topk_warp(sc.exact[half], E, K, lane, myv, myi);
+    float topv[1];
+    int topi[1];
+    topk_warp<1>(sc.exact[half], 128, E, K, lane, topv, topi);
+    const float myv = topv[0];
+    const int myi = topi[0];
     // softmax in the reference's order (refSoftmax.h:23-50), in fp32 as in the GATE task
     const float m = __shfl_sync(0xffffffffu, myv, 0);
     const float ex = (lane < K) ? expf(myv - m) : 0.0f;
@@ -1001,21 +1005,27 @@ __device__ __noinline__ bool gatefix_task(const FdmoeParams& p, SmemCtl& sc, uin
   }
   epi_bar();
   prof_mark(p, sc, etid, 32);
-  // The token row (still in shared memory) goes to its K rows in the owners' expert buffers.
+  // The token row goes to its K rows in the owners' expert buffers.
   if (live) {
+    uint4 xr[FDMOE_MAX_HIDDEN / 8 / 128];
+#pragma unroll
+    for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
+      if (e + i * 128 < H / 8) xr[i] = xsrc[e + i * 128];
     for (int k = 0; k < K; ++k) {
       const uint2 d = sc.fix_dst[half][k];
       if (d.x == 0xffffffffu) continue;
       const int owner = (int)d.x / p.El, le = (int)d.x - owner * p.El;
       uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.peers[owner].packed) +
                                             ((size_t)le * p.cap_rows + d.y) * H);
-      for (int v = e; v < H / 8; v += 128) dst[v] = sc.xrow[half][v];
+#pragma unroll
+      for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
+        if (e + i * 128 < H / 8) dst[e + i * 128] = xr[i];
     }
     ptx::fence_proxy_async();  // packed rows are read by TMA
   }
   epi_bar();
   // the rows have been stored (by all threads, before the barrier): count them on their owners
-  if (live && e < K) {
+  if (live && e < K && sc.batch_mt <= (uint32_t)p.MT) {
     const uint2 d = sc.fix_dst[half][e];
     if (d.x != 0xffffffffu) {
       const int owner = (int)d.x / p.El, le = (int)d.x - owner * p.El;

@@ -1,4 +1,4 @@
-"""GPU parity at the edges of the FFN tiles: every token selects the same experts, so that each of them
+"""GPU parity at the edges of the FFN tiles and of the gating rule.  FFN tiles: every token selects the same experts, so that each of them
 holds exactly as many (different) rows as there are tokens, and all others none."""
 import pytest
 
@@ -32,3 +32,11 @@ def test_rows_per_expert_at_the_edges_of_wide_tiles(rows):
 def test_rows_per_expert_at_the_edges_of_row_boxes(rows):
     s, x, gate, w13, w2 = same_experts(rows)
     check_layer(s, x, gate, w13, w2, max_tokens=128)
+
+
+# one token per gating task, two (the last task with one or two), GATE tiles again; on 148 SMs
+@pytest.mark.parametrize("tokens", [1, 2, 147, 148, 149, 150, 295, 296, 297])
+def test_token_counts_at_the_edges_of_the_gating_rule(tokens):
+    s = synth.TINY
+    gate, w13, w2 = synth.make_weights(s, seed=8, std=0.05)
+    check_layer(s, synth.make_tokens(s, tokens, seed=8), gate, w13, w2, max_tokens=300)
