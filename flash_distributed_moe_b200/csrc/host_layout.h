@@ -48,6 +48,7 @@ struct Geometry {
   int max_tokens_max = 0;    // largest over ranks (sizes token-indexed regions)
   int64_t max_tokens_sum = 0;  // all ranks (sizes expert buffers)
   int cap_rows = 0, MT = 0, combine_group = 8;  // combine_group: tokens per COMBINE task
+  int small_groups = 0;  // groups of a launch with so few tokens that it uses smaller ones (CombineGroup)
   uint32_t queue_cap = 0;
 };
 
@@ -83,7 +84,16 @@ inline bool FinishGeometry(Geometry& g, int grid) {
 }
 
 inline size_t CombineGroups(const Geometry& g) {
-  return (size_t)g.max_tokens_max / std::max(1, g.combine_group) + 2;
+  return (size_t)std::max(g.max_tokens_max / std::max(1, g.combine_group), g.small_groups) + 2;
+}
+
+// Tokens per COMBINE task of a launch on one GPU: as many as give every worker one task, `most` at most.
+// The groups of a decode batch all complete at the end, and nothing is left to overlap them with.
+// Whole layer at 128 tokens of the 2048 x 768 shape: 262 us in groups of 8, 258 us in groups of one.
+inline int CombineGroup(int tokens, int grid, int most) {
+  int g = 1;
+  while (g < most && tokens > g * grid) g *= 2;
+  return std::min(g, most);
 }
 
 inline ArenaLayout MakeLayout(const Geometry& g) {

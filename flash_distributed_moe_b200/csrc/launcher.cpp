@@ -225,6 +225,7 @@ cudaError_t MoeKernelLauncher::Init(const void* gateW, const void* w13, const vo
     g_.max_tokens_sum += h.max_tokens;
   }
   g_.combine_group = std::max(1, EnvInt("FLASHMOE_COMBINE_GROUP", 8));
+  if (world == 1) g_.small_groups = std::min(maxTokens, grid_);
   if (!FinishGeometry(g_, grid_)) {
     MOE_ERROR_LOG("maxTokens=%d: more expert-buffer rows than a dispatch word can address", maxTokens);
     FreeAll();
@@ -407,6 +408,7 @@ cudaError_t MoeKernelLauncher::LaunchBf16(const void* tokens, void* output, int 
     CUDA_ERROR_CHECK(MakeTensorMap(encode_, &p.tm_x, tokens, (uint64_t)tokensNum, g_.H,
                                    std::min(p.gate_rows, tokensNum)));
   }
+  if (world_ == 1) p.combine_group = CombineGroup(tokensNum, grid_, g_.combine_group);
   if (p.disp_conc <= 0) {
     // One GPU: every worker may copy rows (the copies are bound by memory writes).  With peers the
     // links set the pace of the dispatch and a third of the workers keeps them busy, while the others

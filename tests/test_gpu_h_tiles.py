@@ -34,9 +34,10 @@ def test_rows_per_expert_at_the_edges_of_row_boxes(rows):
     check_layer(s, x, gate, w13, w2, max_tokens=128)
 
 
-# one token per gating task, two (the last task with one or two), GATE tiles again; on 148 SMs
-@pytest.mark.parametrize("tokens", [1, 2, 147, 148, 149, 150, 295, 296, 297])
+# on 148 SMs: one token per gating task, two (the last task with one or two), GATE tiles again; and one, two,
+# four, eight tokens per COMBINE task
+@pytest.mark.parametrize("tokens", [1, 2, 147, 148, 149, 150, 295, 296, 297, 592, 593])
 def test_token_counts_at_the_edges_of_the_gating_rule(tokens):
     s = synth.TINY
     gate, w13, w2 = synth.make_weights(s, seed=8, std=0.05)
-    check_layer(s, synth.make_tokens(s, tokens, seed=8), gate, w13, w2, max_tokens=300)
+    check_layer(s, synth.make_tokens(s, tokens, seed=8), gate, w13, w2, max_tokens=max(tokens, 300))
