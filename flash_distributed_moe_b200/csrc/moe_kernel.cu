@@ -1237,6 +1237,100 @@ __device__ __forceinline__ void ffn2_epilogue(SmemCtl& sc, uint32_t taddr, uint6
   }
 }
 
+// A (half) tile of up to 64 rows is computed transposed: the weights are the M operand, two blocks of 128,
+// and the rows the N operand, in steps of 16.  As M operand the rows are padded to 128.  What that costs is
+// power: the board's limit holds this kernel's clock down (1.3 GHz of 1.965 measured inside back-to-back
+// launches of 128 tokens, 1.2 to 1.45 GHz at 4096), and MMAs on rows that do not exist take their share of
+// it also where memory sets the pace.  The line is the one up to which rows are loaded in boxes of 16; at 64
+// rows the transposed form has half the MMA cycles.  With peers the other form stays, whose stores over
+// NVLink are whole lines.  Whole layer, padded and transposed: 4096 x 1536 shape at 64 tokens 869 and
+// 780 us, at 2048 tokens 1237 and 1156; 2048 x 768 shape at 16, 128, 333, 4096 tokens 175 and 171, 268 and
+// 249, 302 and 289, 582 and 576.
+// Block b of the weights has its accumulator at column b * kBlockCols; lanes are weight rows.
+constexpr uint32_t kBlockCols = 64;
+template <bool S>
+__device__ __forceinline__ bool transposed(uint32_t rows) { return !S && rows <= 64u; }
+
+// MMAs of one k-block of a (half) tile: A and B as they lie in a stage.
+template <bool S>
+__device__ __forceinline__ void mma_kblock(uint32_t d_tmem, uint32_t rows_smem, uint32_t weights_smem, uint32_t rows,
+                                           bool accumulate) {
+  const uint64_t dr = ptx::make_smem_desc_sw128(rows_smem), dw = ptx::make_smem_desc_sw128(weights_smem);
+  if (transposed<S>(rows)) {
+    const uint32_t idesc = ptx::make_idesc_bf16(128, (rows + 15u) & ~15u);
+    const uint64_t dw1 = ptx::make_smem_desc_sw128(weights_smem + kStageA);
+#pragma unroll
+    for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4) {
+      ptx::umma_bf16(d_tmem, dw + k4 * 2u, dr + k4 * 2u, idesc, accumulate || k4 != 0u);
+      ptx::umma_bf16(d_tmem + kBlockCols, dw1 + k4 * 2u, dr + k4 * 2u, idesc, accumulate || k4 != 0u);
+    }
+  } else {
+#pragma unroll
+    for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4)
+      ptx::umma_bf16(d_tmem, dr + k4 * 2u, dw + k4 * 2u, ptx::make_idesc_bf16(128, 256), accumulate || k4 != 0u);
+  }
+}
+
+// Stores 16 rows of which this lane holds one column: v[r] goes to column `lane` of a 32-column segment of
+// row r, which starts at `ptr` of lane r (0 = no row).  Two neighbouring lanes exchange, so that each
+// writes two columns of every other row: an instruction covers 2 rows x 64 contiguous bytes.
+__device__ __forceinline__ void store_columns16(const float (&v)[16], int lane, unsigned long long ptr) {
+  const bool odd = lane & 1;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float give = odd ? v[2 * i] : v[2 * i + 1], keep = odd ? v[2 * i + 1] : v[2 * i];
+    const float got = __shfl_xor_sync(0xffffffffu, give, 1);
+    const unsigned long long pp = __shfl_sync(0xffffffffu, ptr, 2 * i + (odd ? 1 : 0));
+    if (pp) reinterpret_cast<uint32_t*>(pp)[lane >> 1] = odd ? pack_bf16(got, keep) : pack_bf16(keep, got);
+  }
+}
+
+// Epilogues of transposed tiles.  FFN1: warp h takes every other 16 rows, quadrant q columns 32 q .. 32 q + 31.
+__device__ __forceinline__ void ffn1_columns(const FdmoeParams& p, uint32_t taddr, uint64_t* tmem_empty_bar, int q, int h,
+                                             int lane, uint32_t e, uint32_t j, uint32_t n, uint32_t rows) {
+  const uint32_t tbase = taddr + ((uint32_t)(q * 32) << 16);
+  for (uint32_t r0 = h * 16; r0 < rows; r0 += 32u) {
+    uint32_t g[16], u[16];
+    ptx::tmem_ld_32x16(tbase + r0, g);
+    ptx::tmem_ld_32x16(tbase + kBlockCols + r0, u);
+    ptx::tmem_ld_wait();
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = silu_mul(__uint_as_float(g[i]), __uint_as_float(u[i]));
+    unsigned long long ptr = 0ull;
+    if (lane < 16 && r0 + lane < rows)
+      ptr = reinterpret_cast<unsigned long long>(reinterpret_cast<bf16*>(p.act) +
+                                                 ((size_t)e * p.cap_rows + (size_t)j * 128 + r0 + lane) * p.I +
+                                                 n * FDMOE_TILE_N1 + q * 32);
+    store_columns16(v, lane, ptr);
+  }
+  release_acc(tmem_empty_bar, lane);
+}
+// FFN2: warp h takes block h of the weights (128 result columns).
+__device__ __forceinline__ void ffn2_columns(const FdmoeParams& p, uint32_t taddr, uint64_t* tmem_empty_bar, int q, int h,
+                                             int lane, uint32_t e, uint32_t j, uint32_t n, uint32_t rows) {
+  const uint32_t tbase = taddr + ((uint32_t)(q * 32) << 16) + h * kBlockCols;
+  for (uint32_t r0 = 0; r0 < rows; r0 += 16u) {
+    unsigned long long ptr = 0ull;
+    float weight = 0.f;
+    if (lane < 16 && r0 + lane < rows) {
+      const uint4 mraw = ld_cg_u4(&p.peers[p.rank].meta[(size_t)e * p.cap_rows + (size_t)j * 128 + r0 + lane]);
+      weight = __uint_as_float(mraw.z);
+      ptr = reinterpret_cast<unsigned long long>(reinterpret_cast<bf16*>(p.peers[p.rank].ystage) +
+                                                 ((size_t)mraw.x * p.K + (mraw.y & 0xffu)) * p.H + n * FDMOE_TILE_N2 +
+                                                 h * 128 + q * 32);
+    }
+    uint32_t d[16];
+    ptx::tmem_ld_32x16(tbase + r0, d);
+    ptx::tmem_ld_wait();
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(d[i]) * __shfl_sync(0xffffffffu, weight, i);
+    store_columns16(v, lane, ptr);
+  }
+  release_acc(tmem_empty_bar, lane);
+}
+
 // COMBINE streams the K weighted rows of each token of a group through the
 // shared-memory stage ring with 1-D bulk copies (issued by the TMA warp) in
 // pieces of up to 2048 columns: stage layout [K][piece], the piece's bytes per slot row.
@@ -1591,7 +1685,6 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
   } else if (warp == kWarpMma) {
     {
       const bool elected = ptx::elect_one();
-      constexpr uint32_t idesc256 = ptx::make_idesc_bf16(128, 256);
       constexpr uint32_t idesc128 = ptx::make_idesc_bf16(128, 128);
       uint32_t stage_it = 0, wide_it = 0, tile_it = 0, skips = 0;
       for (uint32_t it = 0;; ++it) {
@@ -1606,7 +1699,8 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           // accumulator may still be read by the previous task's epilogue: the first one then runs
           // ahead, as far as there are stages.
           const uint32_t nkb = (kind == FDMOE_TASK_FFN2) ? nkb2 : nkb1;
-          const bool pair = (t.c & FDMOE_TILE_ROWS) > 128u;
+          const uint32_t rows = t.c & FDMOE_TILE_ROWS;
+          const bool pair = rows > 128u;
           const uint32_t acc0 = tile_it & 1u, aph0 = (tile_it >> 1) & 1u;
           const uint32_t acc1 = acc0 ^ 1u, aph1 = ((tile_it + 1u) >> 1) & 1u;
           tile_it += pair ? 2u : 1u;
@@ -1621,10 +1715,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
             ptx::tcgen05_fence_after();
             if (elected) {
               const uint32_t sa = ptx::smem_u32(stage + s * kWideBytes);
-              const uint64_t da = ptx::make_smem_desc_sw128(sa), db = ptx::make_smem_desc_sw128(sa + 2 * kStageA);
-#pragma unroll
-              for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4)
-                ptx::umma_bf16(tmem_base + acc0 * kAccCols, da + k4 * 2u, db + k4 * 2u, idesc256, (kb | k4) != 0u);
+              mma_kblock<S>(tmem_base + acc0 * kAccCols, sa, sa + 2 * kStageA, min(128u, rows), kb != 0u);
               if (!pair) ptx::umma_commit(&sc.wide_empty[s]);
               if (kb == nkb - 1u) ptx::umma_commit(&sc.tmem_full[acc0]);
             }
@@ -1645,11 +1736,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
                 for (; kb1 <= kb; ++kb1, ++it1) {
                   const uint32_t s1 = it1 % kWideStages;
                   const uint32_t sa = ptx::smem_u32(stage + s1 * kWideBytes);
-                  const uint64_t da = ptx::make_smem_desc_sw128(sa + kStageA);
-                  const uint64_t db = ptx::make_smem_desc_sw128(sa + 2 * kStageA);
-#pragma unroll
-                  for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4)
-                    ptx::umma_bf16(tmem_base + acc1 * kAccCols, da + k4 * 2u, db + k4 * 2u, idesc256, (kb1 | k4) != 0u);
+                  mma_kblock<S>(tmem_base + acc1 * kAccCols, sa + kStageA, sa + 2 * kStageA, rows - 128u, kb1 != 0u);
                   ptx::umma_commit(&sc.wide_empty[s1]);
                 }
                 if (kb == nkb - 1u) ptx::umma_commit(&sc.tmem_full[acc1]);
@@ -1662,7 +1749,6 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
           if (!ok) break;
         } else if (kind == FDMOE_TASK_FFN1 || kind == FDMOE_TASK_FFN2 || kind == FDMOE_TASK_GATE) {
           const uint32_t nkb = (kind == FDMOE_TASK_FFN2) ? nkb2 : nkb1;
-          const uint32_t idesc = (kind == FDMOE_TASK_GATE) ? idesc128 : idesc256;
           const uint32_t acc = tile_it & 1u, aph = (tile_it >> 1) & 1u;
           ++tile_it;
           if (!wait_bar_warp(p, sc, &sc.tmem_empty[acc], aph ^ 1u, FDMOE_ERR_TIMEOUT_TMEM)) break;
@@ -1676,14 +1762,15 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
             ptx::tcgen05_fence_after();
             if (elected) {
               const uint32_t sa = ptx::smem_u32(stage + s * kStageBytes);
-              for (uint32_t i = 0; i < gk; ++i) {
+              if (kind != FDMOE_TASK_GATE) mma_kblock<S>(d_tmem, sa, sa + kStageA, t.c, kb != 0u);
+              for (uint32_t i = 0; kind == FDMOE_TASK_GATE && i < gk; ++i) {
                 // (a GATE stage with two k-blocks: A at 8 KB, B at 16 KB steps)
                 const uint64_t da = ptx::make_smem_desc_sw128(sa + i * (kStageA / 2));
                 const uint64_t db = ptx::make_smem_desc_sw128(sa + kStageA + i * kStageA);
 #pragma unroll
                 for (uint32_t k4 = 0; k4 < FDMOE_TILE_K / 16; ++k4) {
                   // +32 bytes per 16-element k step inside the 128-byte swizzle row
-                  ptx::umma_bf16(d_tmem, da + k4 * 2u, db + k4 * 2u, idesc, (kb | i | k4) != 0u);
+                  ptx::umma_bf16(d_tmem, da + k4 * 2u, db + k4 * 2u, idesc128, (kb | i | k4) != 0u);
                 }
               }
               ptx::umma_commit(&sc.empty_bar[s]);  // frees the stage when the MMAs have read it
@@ -1776,7 +1863,16 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
             if (!landed) break;
             if (p.prof && etid == 0 && hf == 0) pt1 = prof_now();
             ptx::tcgen05_fence_after();
-            ffn1_epilogue(p, sc, taddr, &sc.tmem_empty[acc], q, h, lane, ewarp, e, j + hf, n, hrows);
+            if (transposed<S>(hrows))
+              ffn1_columns(p, taddr, &sc.tmem_empty[acc], q, h, lane, e, j + hf, n, hrows);
+            else
+              ffn1_epilogue(p, sc, taddr, &sc.tmem_empty[acc], q, h, lane, ewarp, e, j + hf, n, hrows);
+          } else if (transposed<S>(hrows)) {
+            landed = epi_vote_all(wait_bar(p, sc, &sc.tmem_full[acc], aph, FDMOE_ERR_TIMEOUT_TMEM));
+            if (!landed) break;
+            if (p.prof && etid == 0 && hf == 0) pt1 = prof_now();
+            ptx::tcgen05_fence_after();
+            ffn2_columns(p, taddr, &sc.tmem_empty[acc], q, h, lane, e, j + hf, n, hrows);
           } else {
             // the row's destination comes from global memory: asked for before the accumulator is waited for
             const YRow y = ffn2_row(p, q, h, lane, e, j + hf, n, hrows);

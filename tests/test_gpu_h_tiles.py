@@ -21,7 +21,7 @@ def same_experts(tokens):
 
 # one m-tile and two; a wide task's second half with one row, part of a box of rows, and full; a wide task
 # of one m-tile behind a full one
-@pytest.mark.parametrize("rows", [128, 129, 200, 255, 256, 257, 384, 385])
+@pytest.mark.parametrize("rows", [128, 129, 191, 192, 193, 200, 255, 256, 257, 320, 384, 385])
 def test_rows_per_expert_at_the_edges_of_wide_tiles(rows):
     s, x, gate, w13, w2 = same_experts(rows)
     check_layer(s, x, gate, w13, w2, max_tokens=rows)
