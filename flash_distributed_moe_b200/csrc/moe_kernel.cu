@@ -541,6 +541,11 @@ __device__ __forceinline__ void rows_landed(const FdmoeParams& p, uint32_t B, in
 // epilogue group runs it next (flag run_round2).  Called by one full warp.
 template <bool S>
 __device__ __forceinline__ void gating_finished(const FdmoeParams& p, SmemCtl* sc, int lane) {
+  if (!S && sc) {  // one rank: nothing to tell and nobody to wait for
+    if (lane == 0) sc->run_round2 = 1u;
+    __syncwarp();
+    return;
+  }
   fence_acqrel<S>();
   uint32_t prev = 0u;
   if (lane < p.world) prev = atom_add<S>(&p.peers[lane].ctl->ranks_gated, 1u);
@@ -1106,10 +1111,10 @@ __device__ __noinline__ void gated_task(const FdmoeParams& p, SmemCtl& sc, int e
     fence_acqrel<false>();
     for (uint32_t idx = 0; idx < mytasks; ++idx)
       st_relaxed<false>(&slots[(t1 + idx) & (uint32_t)p.queue_mask].seq, t1 + idx + 1u);
-    atom_add<false>(&me.ctl->q[1].avail, mytasks);
   }
   epi_bar();
   if (etid == 0) {
+    if (all) atom_add<false>(&me.ctl->q[1].avail, all);
     st_release<false>(&me.ctl->gated_done, 1u);
     maybe_close(p);
   }
