@@ -957,6 +957,8 @@ __device__ __noinline__ bool gatefix_task(const FdmoeParams& p, SmemCtl& sc, uin
     for (uint32_t kb = 0; kb < nkb; kb += kFixBlocks, ++stage_it) {
       const uint32_t s = stage_it % kStages, sph = (stage_it / kStages) & 1u;
       if (!epi_vote_all(wait_bar(p, sc, &sc.full_bar[s], sph, FDMOE_ERR_TIMEOUT_STAGE))) return false;
+      // (past the vote every thread has read the stage before this one)
+      if (kb && etid == 0) ptx::mbar_arrive(&sc.empty_bar[(stage_it - 1u) % kStages]);
       if (etid < E) {  // (E <= 128: the first four warps)
         const uint32_t nb = min((uint32_t)kFixBlocks, nkb - kb);
         const uint8_t* st = stage + s * kStageBytes;
@@ -966,13 +968,19 @@ __device__ __noinline__ bool gatefix_task(const FdmoeParams& p, SmemCtl& sc, uin
         else
           exact_logits<false>(st, xa, xb, (uint32_t)e, nb, acc_a, acc_b);
       }
-      epi_bar();  // every thread has read the stage (and, at the end, the token rows)
-      if (etid == 0) ptx::mbar_arrive(&sc.empty_bar[s]);
     }
+    epi_bar();  // every thread has read the last stage and the token rows
+    if (etid == 0) ptx::mbar_arrive(&sc.empty_bar[(stage_it - 1u) % kStages]);
     if (etid < E) {
       sc.exact[0][e] = acc_a;
       sc.exact[1][e] = acc_b;
     }
+  }
+  uint4 xr[FDMOE_MAX_HIDDEN / 8 / 128];  // the row again, as it is stored (asked for early, used last)
+  if (live) {
+#pragma unroll
+    for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
+      if (e + i * 128 < H / 8) xr[i] = xsrc[e + i * 128];
   }
   epi_bar();
   prof_mark(p, sc, etid, 31);
@@ -1012,10 +1020,6 @@ __device__ __noinline__ bool gatefix_task(const FdmoeParams& p, SmemCtl& sc, uin
   prof_mark(p, sc, etid, 32);
   // The token row goes to its K rows in the owners' expert buffers.
   if (live) {
-    uint4 xr[FDMOE_MAX_HIDDEN / 8 / 128];
-#pragma unroll
-    for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
-      if (e + i * 128 < H / 8) xr[i] = xsrc[e + i * 128];
     for (int k = 0; k < K; ++k) {
       const uint2 d = sc.fix_dst[half][k];
       if (d.x == 0xffffffffu) continue;
@@ -1026,7 +1030,9 @@ __device__ __noinline__ bool gatefix_task(const FdmoeParams& p, SmemCtl& sc, uin
       for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
         if (e + i * 128 < H / 8) dst[e + i * 128] = xr[i];
     }
-    ptx::fence_proxy_async();  // packed rows are read by TMA
+    // (packed rows are read by TMA: the warp that issues the loads fences between the proxies; rows for a
+    // peer are fenced here too)
+    if (S) ptx::fence_proxy_async();
   }
   epi_bar();
   // the rows have been stored (by all threads, before the barrier): count them on their owners
