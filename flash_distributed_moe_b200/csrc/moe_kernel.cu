@@ -166,6 +166,11 @@ __device__ __forceinline__ uint32_t atom_add(uint32_t* p, uint32_t v) {
     asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
   return old;
 }
+__device__ __forceinline__ uint32_t atom_add_acquire(uint32_t* p, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.acquire.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
 template <bool S>
 __device__ __forceinline__ uint32_t atom_exch(uint32_t* p, uint32_t v) {
   uint32_t old;
@@ -393,7 +398,7 @@ __device__ __forceinline__ bool try_pop(const FdmoeParams& p, SmemCtl& sc, int q
   const FdmoePeer& me = p.peers[p.rank];
   FdmoeQueueCtl* q = &me.ctl->q[qi];
   if ((int32_t)ld_relaxed<S>(&q->avail) <= 0) return false;
-  if ((int32_t)atomicSub(&q->avail, 1u) <= 0) {
+  if ((int32_t)atom_add_acquire(&q->avail, 0xffffffffu) <= 0) {
     atomicAdd(&q->avail, 1u);  // others were faster: give the unit back
     return false;
   }
@@ -1104,22 +1109,38 @@ __device__ __noinline__ void gated_task(const FdmoeParams& p, SmemCtl& sc, int e
     sc.q_t0 = all ? atom_add<false>(&me.ctl->q[1].head, all) : 0u;
   }
   epi_bar();
+  // Without batches nobody else publishes on this queue: a consumer that got its unit of the count, raised
+  // behind one fence (and taken with acquire, see try_pop), finds its slot complete, sequence word included.
+  const bool alone = B > (uint32_t)p.MT;
   if (mytasks) {
     const uint32_t t1 = sc.q_t0 + before + inc - mytasks;
     FdmoeSlot* slots = me.slots[1];
+    uint32_t jt = first, n = 0;
     for (uint32_t idx = 0; idx < mytasks; ++idx) {
-      const uint32_t jt = first + (idx / nt1) * step, n = idx % nt1;
       FdmoeSlot* sl = &slots[(t1 + idx) & (uint32_t)p.queue_mask];
-      sl->a = task_word(FDMOE_TASK_FFN1, (uint32_t)etid, n);
-      sl->b = jt;
-      sl->c = min(128u * step, lcnt - jt * 128u) | (step > 1u ? (uint32_t)FDMOE_TILE_WIDE : 0u);
+      const uint32_t a = task_word(FDMOE_TASK_FFN1, (uint32_t)etid, n);
+      const uint32_t c = min(128u * step, lcnt - jt * 128u) | (step > 1u ? (uint32_t)FDMOE_TILE_WIDE : 0u);
+      if (alone) {
+        *reinterpret_cast<uint4*>(sl) = make_uint4(t1 + idx + 1u, a, jt, c);
+      } else {
+        sl->a = a;
+        sl->b = jt;
+        sl->c = c;
+      }
+      if (++n == nt1) {
+        n = 0;
+        jt += step;
+      }
     }
-    fence_acqrel<false>();
-    for (uint32_t idx = 0; idx < mytasks; ++idx)
-      st_relaxed<false>(&slots[(t1 + idx) & (uint32_t)p.queue_mask].seq, t1 + idx + 1u);
+    if (!alone) {
+      fence_acqrel<false>();
+      for (uint32_t idx = 0; idx < mytasks; ++idx)
+        st_relaxed<false>(&slots[(t1 + idx) & (uint32_t)p.queue_mask].seq, t1 + idx + 1u);
+    }
   }
   epi_bar();
   if (etid == 0) {
+    if (alone) fence_acqrel<false>();
     if (all) atom_add<false>(&me.ctl->q[1].avail, all);
     st_release<false>(&me.ctl->gated_done, 1u);
     maybe_close(p);
