@@ -391,13 +391,13 @@ __device__ __forceinline__ FdmoeSlot exit_task() {
   return out;
 }
 
-// Takes the oldest task of queue `qi` of this rank if there is one (single thread).  Returns
-// false when the queue is empty (or on an error, with sc.abort raised).
+// Takes the oldest task of queue `qi` of this rank if there still is one (single thread; the caller has
+// seen the queue's count above zero).  Returns false when others were faster (or on an error, with
+// sc.abort raised).
 template <bool S>
 __device__ __forceinline__ bool try_pop(const FdmoeParams& p, SmemCtl& sc, int qi, FdmoeSlot& out) {
   const FdmoePeer& me = p.peers[p.rank];
   FdmoeQueueCtl* q = &me.ctl->q[qi];
-  if ((int32_t)ld_relaxed<S>(&q->avail) <= 0) return false;
   if ((int32_t)atom_add_acquire(&q->avail, 0xffffffffu) <= 0) {
     atomicAdd(&q->avail, 1u);  // others were faster: give the unit back
     return false;
@@ -438,13 +438,18 @@ __device__ __forceinline__ FdmoeSlot next_task(const FdmoeParams& p, SmemCtl& sc
   uint32_t spins = 0;
   for (;;) {
     if (sc.abort) return exit_task();
-    if (S && try_pop<S>(p, sc, 0, out)) return out;
-    if ((int32_t)ld_relaxed<false>(&ctl->q[2].avail) > 0 && ld_relaxed<false>(&ctl->disp_active) < (uint32_t)p.disp_conc) {
+    // every word the decision rests on, asked for at once: one after the other they are five round trips to
+    // L2, 0.7 us each, before an idle worker sees its task
+    const int32_t n0 = (int32_t)ld_relaxed<S>(&ctl->q[0].avail), n1 = (int32_t)ld_relaxed<S>(&ctl->q[1].avail);
+    const int32_t n2 = (int32_t)ld_relaxed<false>(&ctl->q[2].avail);
+    const uint32_t gates = ld_relaxed<false>(&ctl->gate_next), closed = ld_relaxed<false>(&ctl->closed);
+    if (S && n0 > 0 && try_pop<S>(p, sc, 0, out)) return out;
+    if (n2 > 0 && ld_relaxed<false>(&ctl->disp_active) < (uint32_t)p.disp_conc) {
       if (atomicAdd(&ctl->disp_active, 1u) < (uint32_t)p.disp_conc && try_pop<false>(p, sc, 2, out)) return out;
       atomicSub(&ctl->disp_active, 1u);
     }
-    if (!S && try_pop<S>(p, sc, 0, out)) return out;
-    if (gate_tiles != 0u && ld_relaxed<false>(&ctl->gate_next) < gate_tiles) {
+    if (!S && n0 > 0 && try_pop<S>(p, sc, 0, out)) return out;
+    if (gates < gate_tiles) {
       const uint32_t g = atomicAdd(&ctl->gate_next, 1u);
       if (g < gate_tiles) {
         out.seq = 0;
@@ -462,8 +467,8 @@ __device__ __forceinline__ FdmoeSlot next_task(const FdmoeParams& p, SmemCtl& sc
         return out;
       }
     }
-    if (try_pop<S>(p, sc, 1, out)) return out;
-    if (ld_relaxed<false>(&ctl->closed) != 0u) return exit_task();
+    if (n1 > 0 && try_pop<S>(p, sc, 1, out)) return out;
+    if (closed != 0u) return exit_task();
     if ((++spins & 15u) == 0u) {
       if (ptx::globaltimer_ns() - t0 > p.timeout_ns) {
         raise_error(p, sc, FDMOE_ERR_TIMEOUT_QUEUE, (blockIdx.x << 8));
