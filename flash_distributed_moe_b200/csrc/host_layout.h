@@ -128,6 +128,18 @@ inline ArenaLayout MakeLayout(const Geometry& g) {
   return L;
 }
 
+// Experts with more rows than this get wide FFN tasks (FDMOE_TILE_WIDE) in a launch on one GPU.  Wide tasks are
+// twice as long, and going from narrow to wide stages drains the pipeline, so a launch uses them only if
+// there are about three wide FFN1 tasks per worker.  Whole layer on 148 SMs, narrow only and wide from 129
+// rows on: 16 experts of 4096 x 1536 at 400 tokens (1.0 tasks per worker) 265 and 299 us, at 700 (1.8) 325
+// and 358, at 1300 (3.3) 503 and 484; 2048 x 768 shape at 1800 tokens (2.3) 332 and 350, at 2048 (2.6) 347
+// and 366, at 2500 (3.2) 402 and 396; 4096 x 1536 shape at 2048 tokens (5.2) 1184 and 1115.
+constexpr int kNoWideRows = 1 << 30;
+inline int WideRows(const Geometry& g, int tokens, int grid) {
+  const uint64_t tasks = (uint64_t)tokens * g.K / (2 * FDMOE_TILE_M) * (g.I / FDMOE_TILE_N1);
+  return tasks < 3ull * grid ? kNoWideRows : FDMOE_TILE_M;
+}
+
 // Tokens per gating task of a launch on one GPU.  32, 64 or 128: GATE tiles, the smallest that still
 // gives every SM at most one tile, so that the gate phase spreads over as many SMs as possible.  1 or 2:
 // every token is gated exactly, which saves a small launch the tensor-core gate, the separate dispatch

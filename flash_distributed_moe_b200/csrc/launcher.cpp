@@ -408,6 +408,7 @@ cudaError_t MoeKernelLauncher::LaunchBf16(const void* tokens, void* output, int 
     CUDA_ERROR_CHECK(MakeTensorMap(encode_, &p.tm_x, tokens, (uint64_t)tokensNum, g_.H,
                                    std::min(p.gate_rows, tokensNum)));
   }
+  p.wide_rows = std::max<int>(FDMOE_TILE_M, EnvInt("FLASHMOE_WIDE_ROWS", WideRows(g_, tokensNum, grid_)));
   if (world_ == 1) p.combine_group = CombineGroup(tokensNum, grid_, g_.combine_group);
   if (p.disp_conc <= 0) {
     // One GPU: every worker may copy rows (the copies are bound by memory writes).  With peers the

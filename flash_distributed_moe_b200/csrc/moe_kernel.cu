@@ -6,12 +6,14 @@
 //   GATE     token tile: gate GEMM on tcgen05, top-k, softmax; indices and weights go to global
 //            memory.  Tokens whose leading logits are nearly tied are recomputed by a GATEFIX task
 //            with fp32 FMAs in the reference's accumulation order, so the selection is the
-//            reference's;
+//            reference's.  On one GPU a launch of few tokens has GATEFIX tasks only, which do the
+//            DISPATCH of their tokens too;
 //   DISPATCH the rows of one GATE tile: rows are reserved in the owners' expert buffers, every
 //            token row is brought into shared memory once and goes out as K bulk copies, one per
 //            selected expert, into the owner's buffer (local, or a peer's over NVLink);
-//   FFN1/2   128-row expert tiles on tcgen05 with TMEM accumulators fed by TMA (SwiGLU epilogue;
-//            routing-weight epilogue stored on the token's home rank).  The sender whose rows
+//   FFN1/2   expert tiles of 128 or 256 rows (few rows: transposed, as the N operand) on tcgen05
+//            with TMEM accumulators fed by TMA (SwiGLU epilogue; routing-weight epilogue stored on
+//            the token's home rank).  The sender whose rows
 //            complete a batch of m-tiles of an expert publishes the batch's FFN1 tiles on the
 //            owner's queue; what is left when every rank has gated is published by the owner's
 //            GATED task, expert by expert;
@@ -1084,8 +1086,8 @@ __device__ __noinline__ void gated_task(const FdmoeParams& p, SmemCtl& sc, int e
     ntile = (lcnt + 127u) / 128u;
     first = ((lcnt / 128u) / B) * B;
   }
-  // m-tiles per task (see FDMOE_TILE_WIDE for the reason of the line at 128 rows)
-  const uint32_t step = (!S && lcnt > 128u) ? 2u : 1u;
+  // m-tiles per task (WideRows draws the line)
+  const uint32_t step = (!S && lcnt > (uint32_t)p.wide_rows) ? 2u : 1u;
   const uint32_t mytasks = ((ntile - first + step - 1u) / step) * nt1;
   uint32_t inc = mytasks, inc_tile = ntile;
 #pragma unroll

@@ -55,9 +55,8 @@ enum {
 // The third word of an FFN1 / FFN2 task: valid rows of the tile (up to 128; a wide one's up to 256) and
 // whether it is wide.  A wide task runs two m-tiles of an expert against each block of weights, which
 // brings 64 KB of operands into shared memory for what costs two narrow ones 96 KB.  On one GPU an
-// expert's tasks are wide from 129 rows on: below there is no second m-tile, and from there on both
-// forms were measured (B200, whole layer, narrow and wide): 16384 tokens of the 2048 x 768 shape
-// 1560 and 1513 us, 4096 tokens 551 and 552 us, 2048 tokens of the 4096 x 1536 shape 1226 and 1161 us.
+// expert's tasks are wide from 129 rows on, where there is a second m-tile, if the launch has enough of
+// them (WideRows).  Whole layer, narrow and wide: 16384 tokens of the 2048 x 768 shape 1560 and 1513 us.
 // With peers they stay narrow: a wide task holds both accumulators through its epilogue, whose stores
 // cross NVLink there.
 enum {
@@ -162,6 +161,8 @@ typedef struct {
   int32_t gate_rows;    // tokens per GATE task: 32, 64 or 128 (rows of the 128-row MMA tile that are used); 1 or 2: no
                         // GATE tasks, every token is gated exactly, one or two per task
   int32_t disp_conc;    // DISPATCH tasks worked on at a time
+  int32_t wide_rows;    // experts with more rows than this get wide FFN tasks (at least 128)
+  int32_t pad_wide;
   int32_t batch_mt;     // m-tiles per publication batch; 0 = chosen from the token counts of the launch
   int32_t mode;         // 0 full layer; 2 static tasks only (no gate)
   uint32_t expected_static;  // mode 2: tasks pre-filled by the host

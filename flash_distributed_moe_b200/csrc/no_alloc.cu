@@ -197,6 +197,7 @@ extern "C" int FlashMoeLaunchNoAlloc(const void* gateWeights, const void* ffn1Ex
   p.mode = 0;
   p.epoch = 1;
   p.disp_conc = d->grid;
+  p.wide_rows = WideRows(g, tokensNum, d->grid);
   p.batch_mt = 0;
   p.timeout_ns = 2000ull * 1000000ull;
   p.peer_timeout_ns = p.timeout_ns;

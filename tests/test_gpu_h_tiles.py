@@ -22,7 +22,8 @@ def same_experts(tokens):
 # one m-tile and two; a wide task's second half with one row, part of a box of rows, and full; a wide task
 # of one m-tile behind a full one
 @pytest.mark.parametrize("rows", [128, 129, 191, 192, 193, 200, 255, 256, 257, 320, 384, 385])
-def test_rows_per_expert_at_the_edges_of_wide_tiles(rows):
+def test_rows_per_expert_at_the_edges_of_wide_tiles(rows, monkeypatch):
+    monkeypatch.setenv("FLASHMOE_WIDE_ROWS", "128")
     s, x, gate, w13, w2 = same_experts(rows)
     check_layer(s, x, gate, w13, w2, max_tokens=rows)
 
@@ -41,3 +42,11 @@ def test_token_counts_at_the_edges_of_the_gating_rule(tokens):
     s = synth.TINY
     gate, w13, w2 = synth.make_weights(s, seed=8, std=0.05)
     check_layer(s, synth.make_tokens(s, tokens, seed=8), gate, w13, w2, max_tokens=max(tokens, 300))
+
+
+# wide and narrow tiles in one launch, in turn
+def test_experts_on_both_sides_of_the_wide_line(monkeypatch):
+    monkeypatch.setenv("FLASHMOE_WIDE_ROWS", "128")
+    s = synth.TINY
+    gate, w13, w2 = synth.make_weights(s, seed=9, std=0.05)
+    check_layer(s, synth.make_tokens(s, 1040, seed=9), gate, w13, w2, max_tokens=1040)
