@@ -140,18 +140,22 @@ inline int WideRows(const Geometry& g, int tokens, int grid) {
   return tasks < 3ull * grid ? kNoWideRows : FDMOE_TILE_M;
 }
 
-// Tokens per gating task of a launch on one GPU.  32, 64 or 128: GATE tiles, the smallest that still
-// gives every SM at most one tile, so that the gate phase spreads over as many SMs as possible.  1 or 2:
-// every token is gated exactly, which saves a small launch the tensor-core gate, the separate dispatch
-// and, for nearly tied tokens, the exact gate after all, as long as one wave of workers does it.  Whole
-// layer of the 2048 x 768 shape on 148 SMs, tiles of 32 tokens / one token / two per task: 128 tokens
-// 296 / 265 / 273 us, 148 tokens 299 / 267 / 275, 200 tokens 299 / 288 / 275, 296 tokens 303 / 292 / 278,
-// 333 tokens 301 / 310 / 304, 592 tokens 312 / 340 / 313.
+// Tokens per GATE tile of a launch on one GPU.  32, 64 or 128: the smallest that still gives every SM at most
+// one tile, so that the gate phase spreads over as many SMs as possible.  1 or 2: the tile's task sends its
+// tokens' rows too, which saves a small launch the separate DISPATCH tasks, as long as one wave of
+// workers does it.
 inline int GateRows(int tokens, int grid) {
   if (tokens <= grid) return 1;
   if (tokens <= 2 * grid) return 2;
   if (tokens <= 32 * grid) return 32;
   return tokens <= 64 * grid ? 64 : 128;
+}
+
+// Whether a launch can have GATE tiles of `rows` tokens.  Tiles of one token may publish a GATEFIX task each
+// (larger ones: one per two tokens), which the queues hold for the launches that the rule gives such tiles.
+inline bool GateRowsFit(int rows, int tokens, int grid, int world) {
+  if (rows == 1 || rows == 2) return world == 1 && (rows == 2 || tokens <= grid);
+  return rows == 32 || rows == 64 || rows == 128;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

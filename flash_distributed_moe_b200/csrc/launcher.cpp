@@ -397,14 +397,10 @@ cudaError_t MoeKernelLauncher::LaunchBf16(const void* tokens, void* output, int 
   if (tokensNum > 0 && mode == 0) {
     // the token matrix moves between launches: its TMA descriptor is rebuilt (host-only arithmetic)
     // (with peers: always GATE tiles of 32 tokens, many small tiles let the tensor cores start on the
-    // first rows while later tiles are still being dispatched over NVLink; the dump of the tensor-core
-    // logits needs GATE tiles too)
-    int rows = GateRows(tokensNum, grid_);
-    if (world_ > 1 || (debug_logits_ && rows < 32)) rows = 32;
+    // first rows while later tiles are still being dispatched over NVLink)
+    const int rows = world_ > 1 ? 32 : GateRows(tokensNum, grid_);
     p.gate_rows = EnvInt("FLASHMOE_GATE_ROWS", rows);
-    const bool exact = p.gate_rows == 1 || p.gate_rows == 2;
-    if (exact ? world_ > 1 || debug_logits_ : p.gate_rows != 32 && p.gate_rows != 64 && p.gate_rows != 128)
-      p.gate_rows = rows;
+    if (!GateRowsFit(p.gate_rows, tokensNum, grid_, world_)) p.gate_rows = rows;
     CUDA_ERROR_CHECK(MakeTensorMap(encode_, &p.tm_x, tokens, (uint64_t)tokensNum, g_.H,
                                    std::min(p.gate_rows, tokensNum)));
   }

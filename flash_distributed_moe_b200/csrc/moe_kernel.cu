@@ -6,8 +6,8 @@
 //   GATE     token tile: gate GEMM on tcgen05, top-k, softmax; indices and weights go to global
 //            memory.  Tokens whose leading logits are nearly tied are recomputed by a GATEFIX task
 //            with fp32 FMAs in the reference's accumulation order, so the selection is the
-//            reference's.  On one GPU a launch of few tokens has GATEFIX tasks only, which do the
-//            DISPATCH of their tokens too;
+//            reference's.  On one GPU a launch of few tokens has GATE tiles of one or two, which do
+//            the DISPATCH of their tokens too;
 //   DISPATCH the rows of one GATE tile: rows are reserved in the owners' expert buffers, every
 //            token row is brought into shared memory once and goes out as K bulk copies, one per
 //            selected expert, into the owner's buffer (local, or a peer's over NVLink);
@@ -87,7 +87,7 @@ struct __align__(64) SmemCtl {
   uint32_t q_total;
   uint32_t prof_n;
   uint32_t n_flagged;
-  uint32_t pre[16];  // GATED scratch: per-warp totals
+  uint32_t pre[16];  // GATED scratch: per-warp totals; GATE tile of up to two tokens: their near-ties
   uint32_t run_round2;  // set by a task body that found this rank's GATED round due: the group runs it next
   uint32_t batch_mt;    // m-tiles per publication batch of this launch (identical on all ranks)
   uint32_t tokens_all;  // tokens of all ranks this launch
@@ -108,11 +108,13 @@ struct __align__(64) SmemCtl {
       uint8_t lpos[FDMOE_GATE_TOKENS][FDMOE_MAX_TOPK];
     };
     struct {
-      // GATEFIX task scratch: two token rows as fp32, later their exact logits and destinations
+      // GATEFIX task scratch: two token rows as fp32, later their logits and destinations (a GATE tile of
+      // up to two tokens has the latter too)
       union {
         float xrow[2][FDMOE_MAX_HIDDEN];
         struct {
-          float exact[2][128];
+          float logits[2][128];
+          uint8_t cand[2][32];                  // experts that a nearly tied token may select
           uint2 fix_dst[2][FDMOE_MAX_TOPK];     // {expert, row in the owner's buffers} of each slot, or {~0, 0}
         };
       };
@@ -139,7 +141,8 @@ __device__ __forceinline__ const FdmoeParams& task_params(const SmemCtl& sc) {
 
 constexpr int kSmemBytes = kStages * kStageBytes + (int)sizeof(SmemCtl) + 1024;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA exceeds the sm_100 limit");
-static_assert(offsetof(SmemCtl, xrow) % 16 == 0 && offsetof(SmemCtl, logit_tile) % 16 == 0 && (132 * 4) % 16 == 0,
+static_assert(offsetof(SmemCtl, xrow) % 16 == 0 && offsetof(SmemCtl, logits) % 16 == 0 &&
+                  offsetof(SmemCtl, logit_tile) % 16 == 0 && (132 * 4) % 16 == 0,
               "vector accesses to the gate scratch need 16-byte alignment");
 static_assert(offsetof(SmemCtl, store_stage) % 16 == 0, "store staging must keep 16-byte alignment");
 static_assert(offsetof(SmemCtl, full_bar) % 8 == 0 && offsetof(SmemCtl, ring) % 16 == 0, "barrier / ring alignment");
@@ -455,17 +458,9 @@ __device__ __forceinline__ FdmoeSlot next_task(const FdmoeParams& p, SmemCtl& sc
       const uint32_t g = atomicAdd(&ctl->gate_next, 1u);
       if (g < gate_tiles) {
         out.seq = 0;
-        if (p.gate_rows <= 2) {
-          // few tokens: gated exactly, one or two per task (GateRows draws the line)
-          const uint32_t t = g * (uint32_t)p.gate_rows;
-          out.a = FDMOE_TASK_GATEFIX;
-          out.b = t;
-          out.c = (p.gate_rows == 2 && t + 1u < (uint32_t)p.T) ? t + 1u : 0xffffffffu;
-        } else {
-          out.a = FDMOE_TASK_GATE;
-          out.b = g;
-          out.c = 0;
-        }
+        out.a = FDMOE_TASK_GATE;
+        out.b = g;
+        out.c = 0;
         return out;
       }
     }
@@ -644,6 +639,12 @@ __device__ __forceinline__ void topk_warp(const float* r0, int pitch, int E, int
   }
 }
 
+// Gap below which two logits of a token count as nearly tied, `top` its largest logit (see gate_epilogue).
+__device__ __forceinline__ float tie_gap(const FdmoeParams& p, float top) {
+  return 3e-8f * (float)p.H * fmaxf(1.0f, fabsf(top));
+}
+constexpr int kTieTop = 9;  // leading logits that are tested, one more than the largest top-k
+
 // Epilogue of a GATE task (256 threads).  The accumulator holds the logits of
 // 128 tokens (TMEM lanes) x 128 experts (columns) as computed by the tensor
 // cores, whose accumulation order is not the reference's.  Measured on B200 the
@@ -662,7 +663,7 @@ __device__ __noinline__ void gate_epilogue(const FdmoeParams& p, SmemCtl& sc, ui
   const int E = p.E, K = p.K;
   const int t0 = (int)tile * p.gate_rows;
   const int nt = min(p.gate_rows, p.T - t0);
-  const int kk = min(E, 9);
+  const int kk = min(E, kTieTop);
   const int npass = p.gate_rows / 32;
 
   if (etid < 128) sc.cnt[etid] = 0;
@@ -720,7 +721,7 @@ __device__ __noinline__ void gate_epilogue(const FdmoeParams& p, SmemCtl& sc, ui
   if (etid < FDMOE_GATE_TOKENS) {
     bool tie = false;
     if (etid < nt) {
-      const float tau = 3e-8f * (float)p.H * fmaxf(1.0f, fabsf(sc.top_v[etid][0]));
+      const float tau = tie_gap(p, sc.top_v[etid][0]);
       for (int j = 0; j + 1 < kk; ++j) tie |= (sc.top_v[etid][j] - sc.top_v[etid][j + 1]) < tau;
       if (tie) sc.flagged[atomicAdd(&sc.n_flagged, 1u)] = (uint32_t)etid;
     }
@@ -941,18 +942,245 @@ __device__ __forceinline__ void exact_logits(const uint8_t* stage, const float* 
   }
 }
 
-// Up to two tokens gated exactly: all E logits with fp32 FMAs in the reference's order, then top-k,
-// softmax, row reservation and the dispatch of the tokens' K rows, i.e. everything GATE and DISPATCH do
-// for the other tokens.  Published by GATE for tokens whose leading tensor-core logits were nearly tied;
-// in launches with few tokens claimed from the gate counter instead of GATE tiles.
+// A token's row in registers, as it is stored: 128 threads, thread e holds 16-byte pieces e, e + 128, ...
+struct TokenRow {
+  uint4 v[FDMOE_MAX_HIDDEN / 8 / 128];
+};
+__device__ __forceinline__ TokenRow load_row(const FdmoeParams& p, uint32_t tok, int e) {
+  TokenRow x;
+  const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.x) + (size_t)tok * p.H);
+#pragma unroll
+  for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
+    if (e + i * 128 < p.H / 8) x.v[i] = src[e + i * 128];
+  return x;
+}
+
+// A nearly tied token of a GATE tile of one or two: the exact logits of the experts it may select, up to 32 of
+// them, one per lane (fp32 FMAs, k ascending, as exact_logits).  `rows` holds the token's row and behind it the
+// experts' gate rows, 16 bytes apart.  A chain of H dependent FMAs of four cycles is the floor.
+__device__ __forceinline__ float exact_logit(const uint8_t* rows, int H, uint32_t lane_row) {
+  const uint4* x = reinterpret_cast<const uint4*>(rows);
+  const uint4* w = reinterpret_cast<const uint4*>(rows + (size_t)H * 2 + (size_t)lane_row * (H * 2 + 16));
+  float acc = 0.f;
+#pragma unroll 8
+  for (int c = 0; c < H / 8; ++c) {
+    const uint4 xv = x[c], wv = w[c];
+    acc = fmaf(bf16_lo(xv.x), bf16_lo(wv.x), acc);
+    acc = fmaf(bf16_hi(xv.x), bf16_hi(wv.x), acc);
+    acc = fmaf(bf16_lo(xv.y), bf16_lo(wv.y), acc);
+    acc = fmaf(bf16_hi(xv.y), bf16_hi(wv.y), acc);
+    acc = fmaf(bf16_lo(xv.z), bf16_lo(wv.z), acc);
+    acc = fmaf(bf16_hi(xv.z), bf16_hi(wv.z), acc);
+    acc = fmaf(bf16_lo(xv.w), bf16_lo(wv.w), acc);
+    acc = fmaf(bf16_hi(xv.w), bf16_hi(wv.w), acc);
+  }
+  return acc;
+}
+constexpr uint32_t kHalfStages = kStages / 2 * kStageBytes;  // what exact_logit's rows of one token may take
+__device__ __forceinline__ uint32_t max_candidates(int H) {
+  return min(32u, (kHalfStages - (uint32_t)H * 2u) / ((uint32_t)H * 2u + 16u));
+}
+constexpr uint32_t kManyTied = 0xffffffffu;  // more candidates than that: the token goes to a GATEFIX task
+
+// Top-k, softmax, row reservation and the dispatch of the K rows of up to two tokens whose logits lie in
+// sc.logits, one half of the group per token (`tok` is this half's, if `live`; `x` its row).  What GATE and
+// DISPATCH do for the tokens of a larger tile, with the same results bit for bit.
+// `Check`: the logits are the tensor cores'.  A nearly tied token's K largest exact logits are among those of
+// the experts whose tensor-core logit is at most the gap below its K-th largest one; these are recomputed here,
+// with the gate rows in the stages, which are free while this task runs.  (A GATEFIX task instead costs
+// two queue hand-overs and all E logits; at 128 tokens of the 2048 x 768 shape two or three tokens are nearly tied
+// and the first FFN tile starts behind them.)  Called by the whole group, behind a barrier.
+template <bool S, bool Check>
+__device__ __forceinline__ void route_tokens(const FdmoeParams& p, SmemCtl& sc, uint8_t* stage, int etid, int ewarp,
+                                             int lane, uint32_t tok, bool live, bool two, const TokenRow& x) {
+  const int H = p.H, E = p.E, K = p.K;
+  const int half = etid >> 7, e = etid & 127;
+  const bool mine = live && (ewarp & 3) == 0;
+  float topv[1] = {0.f};
+  int topi[1] = {0};
+  uint32_t tie_a = 0u, tie_b = 0u;
+  if (mine) topk_warp<1>(sc.logits[half], 128, E, Check ? min(E, kTieTop) : K, lane, topv, topi);
+  if (Check) {
+    if (mine) {
+      const float m = __shfl_sync(0xffffffffu, topv[0], 0), kth = __shfl_sync(0xffffffffu, topv[0], K - 1);
+      const float next = __shfl_down_sync(0xffffffffu, topv[0], 1), gap = tie_gap(p, m);
+      uint32_t n = 0u;
+      if (__any_sync(0xffffffffu, lane + 1 < min(E, kTieTop) && topv[0] - next < gap)) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int c = lane + 32 * i;
+          const bool in = c < E && sc.logits[half][c] >= kth - gap;
+          const uint32_t all = __ballot_sync(0xffffffffu, in);
+          const uint32_t pos = n + __popc(all & ((1u << lane) - 1u));
+          if (in && pos < 32u) sc.cand[half][pos] = (uint8_t)c;
+          n += __popc(all);
+        }
+        // (logits that are not finite are left to GATEFIX too)
+        if (n > max_candidates(H) || !(fabsf(m) < INFINITY) || !(fabsf(kth) < INFINITY)) n = kManyTied;
+      }
+      if (lane == 0) sc.pre[half] = n;
+    }
+    epi_bar();
+    tie_a = sc.pre[0];
+    tie_b = two ? sc.pre[1] : 0u;
+    const bool in_a = tie_a != 0u && tie_a != kManyTied, in_b = tie_b != 0u && tie_b != kManyTied;
+    if (in_a || in_b) {
+      const uint32_t n = half ? tie_b : tie_a;
+      const bool exact = half ? in_b : in_a;
+      uint8_t* rows = stage + half * kHalfStages;
+      if (exact) {
+        const uint4* gate = reinterpret_cast<const uint4*>(p.gate_w);
+        for (uint32_t r = 0; r < n; ++r)
+          for (int c = e; c < H / 8; c += 128)
+            ptx::cp_async16(rows + (size_t)H * 2 + (size_t)r * (H * 2 + 16) + c * 16,
+                            gate + (size_t)sc.cand[half][r] * (H / 8) + c);
+#pragma unroll
+        for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
+          if (e + i * 128 < H / 8) reinterpret_cast<uint4*>(rows)[e + i * 128] = x.v[i];
+        ptx::cp_async_wait_all();
+      }
+      epi_bar();
+      if (mine && exact) {
+        const float acc = exact_logit(rows, H, min((uint32_t)lane, n - 1u));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sc.logits[half][lane + 32 * i] = -INFINITY;
+        __syncwarp();
+        if ((uint32_t)lane < n) sc.logits[half][sc.cand[half][lane]] = acc;
+        __syncwarp();
+        topk_warp<1>(sc.logits[half], 128, E, K, lane, topv, topi);
+      }
+    }
+  }
+  const float myv = topv[0];
+  const int myi = topi[0];
+  if (mine) {
+    const float m = __shfl_sync(0xffffffffu, myv, 0);
+    const bool later = (half ? tie_b : tie_a) == kManyTied;
+    // softmax in the reference's order (refSoftmax.h:23-50), in fp32 as in gate_epilogue
+    const float ex = (lane < K) ? expf(myv - m) : 0.0f;
+    float sum = 1.0f;
+    for (int j = 1; j < K; ++j) sum += __shfl_sync(0xffffffffu, ex, j);
+    if (lane < K) sc.fix_dst[half][lane] = make_uint2(0xffffffffu, 0u);
+    if (lane < K && !later) {
+      const float w = ex / sum;
+      const int owner = myi / p.El, le = myi - owner * p.El;
+      uint32_t pos;
+      if (S && owner != p.rank)
+        pos = atom_add<true>(&p.peers[owner].expert_cnt[le], 1u);
+      else
+        pos = atom_add<false>(&p.peers[owner].expert_cnt[le], 1u);
+      if (pos >= (uint32_t)p.cap_rows) {
+        raise_error(p, sc, FDMOE_ERR_ROW_OVERFLOW, (uint32_t)myi);
+      } else {
+        const size_t rowg = (size_t)le * p.cap_rows + pos;
+        sc.fix_dst[half][lane] = make_uint2((uint32_t)myi, pos);
+        p.topk_idx[(size_t)tok * K + lane] = myi;
+        p.topk_w[(size_t)tok * K + lane] = w;
+        *reinterpret_cast<uint4*>(&p.peers[owner].meta[rowg]) =
+            make_uint4(tok, (uint32_t)((p.rank << 8) | lane), __float_as_uint(w), 0u);
+      }
+    }
+  }
+  epi_bar();
+  prof_mark(p, sc, etid, 32);
+  uint32_t routed = two ? 2u : 1u;
+  if (Check) {
+    ptx::fence_proxy_async();  // (the stages may have been used: they go back to TMA)
+    const bool fix_a = tie_a == kManyTied, fix_b = tie_b == kManyTied;
+    routed -= (uint32_t)fix_a + (uint32_t)fix_b;
+    if (etid == 0 && (fix_a || fix_b) && !sc.abort) {  // (this thread's tok is the first token)
+      queue_push<false>(p, p.peers[p.rank], 0, 1u, [&](uint32_t, uint32_t& a, uint32_t& b, uint32_t& c) {
+        a = FDMOE_TASK_GATEFIX;
+        b = fix_a ? tok : tok + 1u;
+        c = (fix_a && fix_b) ? tok + 1u : 0xffffffffu;
+      });
+    }
+  }
+  // The token row goes to its K rows in the owners' expert buffers.
+  if (live) {
+    for (int k = 0; k < K; ++k) {
+      const uint2 d = sc.fix_dst[half][k];
+      if (d.x == 0xffffffffu) continue;
+      const int owner = (int)d.x / p.El, le = (int)d.x - owner * p.El;
+      uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.peers[owner].packed) +
+                                            ((size_t)le * p.cap_rows + d.y) * H);
+#pragma unroll
+      for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
+        if (e + i * 128 < H / 8) dst[e + i * 128] = x.v[i];
+    }
+    // (packed rows are read by TMA: the warp that issues the loads fences between the proxies; rows for a
+    // peer are fenced here too)
+    if (S) ptx::fence_proxy_async();
+  }
+  epi_bar();
+  // the rows have been stored (by all threads, before the barrier): count them on their owners
+  if (live && e < K && sc.batch_mt <= (uint32_t)p.MT) {
+    const uint2 d = sc.fix_dst[half][e];
+    if (d.x != 0xffffffffu) {
+      const int owner = (int)d.x / p.El, le = (int)d.x - owner * p.El;
+      if (S && owner != p.rank) {
+        fence_acqrel<true>();
+        rows_landed<true>(p, sc.batch_mt, owner, (uint32_t)le, d.y, 1u);
+      } else {
+        fence_acqrel<false>();
+        rows_landed<false>(p, sc.batch_mt, owner, (uint32_t)le, d.y, 1u);
+      }
+    }
+  }
+  epi_bar();
+  if (ewarp == 0) count_gated<S>(p, sc, lane, routed);
+}
+
+// Epilogue of a GATE tile of one or two tokens (launches of few tokens on one GPU, see GateRows): the tile's
+// MMAs are those of a larger tile, so a token's logits, and with them its routing weights, have the same bits
+// at any number of tokens.  The task sends the rows itself, without a DISPATCH task.
+template <bool S>
+__device__ __noinline__ void gate_few_epilogue(const FdmoeParams& p, SmemCtl& sc, uint8_t* stage, uint32_t taddr,
+                                               uint64_t* tmem_empty_bar, int q, int h, int lane, int etid, int ewarp,
+                                               uint32_t tile) {
+  const uint32_t t0 = tile * (uint32_t)p.gate_rows;
+  const bool two = p.gate_rows == 2 && t0 + 1u < (uint32_t)p.T;
+  const uint32_t half = (uint32_t)etid >> 7;
+  const bool live = half == 0u || two;
+  const TokenRow x = load_row(p, live ? t0 + half : t0, etid & 127);  // (used last)
+  if (q == 0) {  // TMEM lanes 0 and 1 hold the tokens
+    uint32_t v[32];
+    const uint32_t tb = taddr + h * 64;
+#pragma unroll
+    for (int c2 = 0; c2 < 2; ++c2) {
+      ptx::tmem_ld_32x32(tb + c2 * 32, v);
+      ptx::tmem_ld_wait();
+      if (lane < (two ? 2 : 1)) {
+        float* dst = &sc.logits[lane][h * 64 + c2 * 32];
+#pragma unroll
+        for (int c = 0; c < 32; c += 4)
+          *reinterpret_cast<uint4*>(dst + c) = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        if (p.debug_logits) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c)
+            p.debug_logits[(size_t)(t0 + lane) * 128 + h * 64 + c2 * 32 + c] = __uint_as_float(v[c]);
+        }
+      }
+    }
+  }
+  ptx::tcgen05_fence_before();
+  __syncwarp();
+  if (lane == 0) ptx::mbar_arrive(tmem_empty_bar);
+  epi_bar();
+  prof_mark(p, sc, etid, 31);
+  route_tokens<S, true>(p, sc, stage, etid, ewarp, lane, t0 + half, live, two, x);
+}
+
+// Up to two tokens whose leading tensor-core logits were nearly tied: all E logits with fp32 FMAs in the
+// reference's order, then what is left of GATE and DISPATCH.  Published by GATE tasks.
 template <bool S>
 __device__ __noinline__ bool gatefix_task(const FdmoeParams& p, SmemCtl& sc, uint8_t* stage, uint32_t& stage_it,
                                           int etid, int ewarp, int lane, uint32_t tok_a, uint32_t tok_b) {
-  const int H = p.H, E = p.E, K = p.K;
+  const int H = p.H, E = p.E;
   const int half = etid >> 7, e = etid & 127;
   const uint32_t tok = half ? tok_b : tok_a;
   const bool two = tok_b != 0xffffffffu, live = half == 0 || two;
-  const uint4* xsrc = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.x) + (size_t)(live ? tok : 0u) * H);
+  const uint4* xsrc = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.x) + (size_t)(live ? tok : tok_a) * H);
   if (live) {
     float4* dst = reinterpret_cast<float4*>(sc.xrow[half]);
     for (int v = e; v < H / 8; v += 128) {
@@ -984,85 +1212,14 @@ __device__ __noinline__ bool gatefix_task(const FdmoeParams& p, SmemCtl& sc, uin
     epi_bar();  // every thread has read the last stage and the token rows
     if (etid == 0) ptx::mbar_arrive(&sc.empty_bar[(stage_it - 1u) % kStages]);
     if (etid < E) {
-      sc.exact[0][e] = acc_a;
-      sc.exact[1][e] = acc_b;
+      sc.logits[0][e] = acc_a;
+      sc.logits[1][e] = acc_b;
     }
   }
-  uint4 xr[FDMOE_MAX_HIDDEN / 8 / 128];  // the row again, as it is stored (asked for early, used last)
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
-      if (e + i * 128 < H / 8) xr[i] = xsrc[e + i * 128];
-  }
+  const TokenRow x = load_row(p, live ? tok : tok_a, e);  // the row again, as it is stored (used last)
   epi_bar();
   prof_mark(p, sc, etid, 31);
-  if (live && (ewarp & 3) == 0) {
-    float topv[1];
-    int topi[1];
-    topk_warp<1>(sc.exact[half], 128, E, K, lane, topv, topi);
-    const float myv = topv[0];
-    const int myi = topi[0];
-    // softmax in the reference's order (refSoftmax.h:23-50), in fp32 as in the GATE task
-    const float m = __shfl_sync(0xffffffffu, myv, 0);
-    const float ex = (lane < K) ? expf(myv - m) : 0.0f;
-    float sum = 1.0f;
-    for (int j = 1; j < K; ++j) sum += __shfl_sync(0xffffffffu, ex, j);
-    if (lane < K) {
-      const float w = ex / sum;
-      const int owner = myi / p.El, le = myi - owner * p.El;
-      uint32_t pos;
-      if (S && owner != p.rank)
-        pos = atom_add<true>(&p.peers[owner].expert_cnt[le], 1u);
-      else
-        pos = atom_add<false>(&p.peers[owner].expert_cnt[le], 1u);
-      sc.fix_dst[half][lane] = make_uint2(0xffffffffu, 0u);
-      if (pos >= (uint32_t)p.cap_rows) {
-        raise_error(p, sc, FDMOE_ERR_ROW_OVERFLOW, (uint32_t)myi);
-      } else {
-        const size_t rowg = (size_t)le * p.cap_rows + pos;
-        sc.fix_dst[half][lane] = make_uint2((uint32_t)myi, pos);
-        p.topk_idx[(size_t)tok * K + lane] = myi;
-        p.topk_w[(size_t)tok * K + lane] = w;
-        *reinterpret_cast<uint4*>(&p.peers[owner].meta[rowg]) =
-            make_uint4(tok, (uint32_t)((p.rank << 8) | lane), __float_as_uint(w), 0u);
-      }
-    }
-  }
-  epi_bar();
-  prof_mark(p, sc, etid, 32);
-  // The token row goes to its K rows in the owners' expert buffers.
-  if (live) {
-    for (int k = 0; k < K; ++k) {
-      const uint2 d = sc.fix_dst[half][k];
-      if (d.x == 0xffffffffu) continue;
-      const int owner = (int)d.x / p.El, le = (int)d.x - owner * p.El;
-      uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.peers[owner].packed) +
-                                            ((size_t)le * p.cap_rows + d.y) * H);
-#pragma unroll
-      for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
-        if (e + i * 128 < H / 8) dst[e + i * 128] = xr[i];
-    }
-    // (packed rows are read by TMA: the warp that issues the loads fences between the proxies; rows for a
-    // peer are fenced here too)
-    if (S) ptx::fence_proxy_async();
-  }
-  epi_bar();
-  // the rows have been stored (by all threads, before the barrier): count them on their owners
-  if (live && e < K && sc.batch_mt <= (uint32_t)p.MT) {
-    const uint2 d = sc.fix_dst[half][e];
-    if (d.x != 0xffffffffu) {
-      const int owner = (int)d.x / p.El, le = (int)d.x - owner * p.El;
-      if (S && owner != p.rank) {
-        fence_acqrel<true>();
-        rows_landed<true>(p, sc.batch_mt, owner, (uint32_t)le, d.y, 1u);
-      } else {
-        fence_acqrel<false>();
-        rows_landed<false>(p, sc.batch_mt, owner, (uint32_t)le, d.y, 1u);
-      }
-    }
-  }
-  epi_bar();
-  if (ewarp == 0) count_gated<S>(p, sc, lane, (tok_b != 0xffffffffu) ? 2u : 1u);
+  route_tokens<S, false>(p, sc, stage, etid, ewarp, lane, tok, live, two, x);
   return true;
 }
 
@@ -1856,6 +2013,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
   } else if (warp >= kWarpEpi0) {
     const int etid = tid - kWarpEpi0 * 32, ewarp = warp - kWarpEpi0;
     const int q = warp & 3, h = ewarp >> 2;
+    const bool few_gated = !S && p.gate_rows <= 2;  // GATE tiles send their tokens' rows themselves
     uint32_t tile_it = 0, done_it = 0, stage_it = 0;
     for (uint32_t it = 0;; ++it) {
       const uint32_t r = it % kRing, ph = (it / kRing) & 1u;
@@ -1875,7 +2033,11 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
         if (!epi_vote_all(wait_bar(p, sc, &sc.tmem_full[acc], aph, FDMOE_ERR_TIMEOUT_TMEM))) break;
         if (p.prof && etid == 0) pt1 = prof_now();
         ptx::tcgen05_fence_after();
-        gate_epilogue<S>(task_params(sc), sc, tmem_base + acc * kAccCols, &sc.tmem_empty[acc], q, h, lane, etid, ewarp, j);
+        if (few_gated)
+          gate_few_epilogue<S>(task_params(sc), sc, stage, tmem_base + acc * kAccCols, &sc.tmem_empty[acc], q, h, lane, etid,
+                               ewarp, j);
+        else
+          gate_epilogue<S>(task_params(sc), sc, tmem_base + acc * kAccCols, &sc.tmem_empty[acc], q, h, lane, etid, ewarp, j);
       } else if (kind == FDMOE_TASK_DISPATCH) {
         if (!dispatch_task<S>(task_params(sc), sc, stage, stage_it, etid, ewarp, lane, j, rows)) break;
         if (etid == 0) {
@@ -2012,7 +2174,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
       } else {
         if (etid == 0) raise_error(p, sc, FDMOE_ERR_BAD_TASK, t.a);
       }
-      if (kind == FDMOE_TASK_DISPATCH || kind == FDMOE_TASK_GATEFIX) {
+      if (kind == FDMOE_TASK_DISPATCH || kind == FDMOE_TASK_GATEFIX || (few_gated && kind == FDMOE_TASK_GATE)) {
         // the task may have found this rank's GATED round due: run it here and now
         epi_bar();
         const bool r2 = sc.run_round2 != 0u;

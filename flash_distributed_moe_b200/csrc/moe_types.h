@@ -36,7 +36,7 @@ enum {
   FDMOE_TASK_EXIT = 7,
   FDMOE_TASK_GATE = 8,     // (token tile): gate GEMM, top-k, softmax, row reservation
   FDMOE_TASK_DISPATCH = 9, // (first token, count): copies the tokens' rows into the owners' expert buffers
-  FDMOE_TASK_GATEFIX = 10, // (token, token): exact fp32 gate of nearly tied tokens (or of all, if few) and their dispatch
+  FDMOE_TASK_GATEFIX = 10, // (token, token): exact fp32 gate of nearly tied tokens and their dispatch
 };
 
 // Status codes written by the kernel (first error wins).
@@ -158,8 +158,8 @@ typedef struct {
   int32_t MT;           // cap_rows / 128
   int32_t queue_mask;   // capacity - 1 of either queue (capacity is a power of two)
   int32_t combine_group;  // tokens per COMBINE task
-  int32_t gate_rows;    // tokens per GATE task: 32, 64 or 128 (rows of the 128-row MMA tile that are used); 1 or 2: no
-                        // GATE tasks, every token is gated exactly, one or two per task
+  int32_t gate_rows;    // tokens per GATE task: 1, 2, 32, 64 or 128 (rows of the 128-row MMA tile that are used); tasks
+                        // of 1 or 2 (one GPU) dispatch their tokens too
   int32_t disp_conc;    // DISPATCH tasks worked on at a time
   int32_t wide_rows;    // experts with more rows than this get wide FFN tasks (at least 128)
   int32_t pad_wide;
