@@ -545,7 +545,8 @@ __device__ __forceinline__ void rows_landed(const FdmoeParams& p, uint32_t B, in
 // The routing of every token of this rank is decided and its rows have landed on their owners:
 // tell every rank.  Whoever brings a rank's count to the world size hands it the GATED task (its
 // row counts are final); if that is the caller's own rank and `sc` is given, the caller's
-// epilogue group runs it next (flag run_round2).  Called by one full warp.
+// epilogue group runs it next (flag run_round2).  Called by one full warp, ordered after what its lane 0 has
+// acquired.
 template <bool S>
 __device__ __forceinline__ void gating_finished(const FdmoeParams& p, SmemCtl* sc, int lane) {
   if (!S && sc) {  // one rank: nothing to tell and nobody to wait for
@@ -558,26 +559,31 @@ __device__ __forceinline__ void gating_finished(const FdmoeParams& p, SmemCtl* s
   if (lane < p.world) prev = atom_add<S>(&p.peers[lane].ctl->ranks_gated, 1u);
   const bool last = lane < p.world && prev == (uint32_t)p.world - 1u;
   if (last) {
-    if (sc && lane == p.rank)
+    if (sc && lane == p.rank) {
+      fence_acqrel<S>();  // acquires what the other ranks counted behind their fences
       sc->run_round2 = 1u;
-    else
+    } else {
       queue_push_rank<S>(p, lane, 0, 1u, [](uint32_t, uint32_t& a, uint32_t& b, uint32_t& c) {
         a = FDMOE_TASK_GATED;
         b = 0;
         c = 0;
       });
+    }
   }
   __syncwarp();
 }
 
-// Counts `n` tokens of this rank as gated; the caller has landed their rows.  Called by one full warp.
+// Counts `n` tokens of this rank as gated; the caller has landed their rows.  The count releases them and
+// acquires those of every worker counted before: the group barriers behind it carry that order on to the
+// threads of the GATED round, which read every worker's row counts.  Called by one full warp.
 template <bool S>
 __device__ __forceinline__ void count_gated(const FdmoeParams& p, SmemCtl& sc, int lane, uint32_t n) {
   uint32_t done = 0u;
   if (lane == 0) {
     fence_acqrel<false>();
-    done = atomicAdd(&p.peers[p.rank].ctl->gated_tokens, n) + n;
+    done = atom_add_acquire(&p.peers[p.rank].ctl->gated_tokens, n) + n;
   }
+  __syncwarp();
   done = __shfl_sync(0xffffffffu, done, 0);
   if (n && done == (uint32_t)p.T) gating_finished<S>(p, &sc, lane);
 }
@@ -1234,8 +1240,8 @@ __device__ __noinline__ void gated_task(const FdmoeParams& p, SmemCtl& sc, int e
   const int lane = etid & 31, w = etid >> 5;
   const uint32_t B = sc.batch_mt;
   const uint32_t nt1 = (uint32_t)(p.I / FDMOE_TILE_N1);
-  // (the caller observed every rank's gating count with an atomic or took this task from the queue
-  // with an acquire load; order this thread's reads after that)
+  // (a thread of this worker has acquired every rank's gating count, see count_gated and gating_finished, or the
+  // queue slot of this task; the barriers since then order this thread's reads after that)
   fence_acqrel<S>();
   uint32_t lcnt = 0, ntile = 0, first = 0;
   if (etid < p.El) {
