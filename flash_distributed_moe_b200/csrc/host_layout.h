@@ -49,15 +49,15 @@ struct Geometry {
   int64_t max_tokens_sum = 0;  // all ranks (sizes expert buffers)
   int cap_rows = 0, MT = 0, combine_group = 8;  // combine_group: tokens per COMBINE task
   int small_groups = 0;  // groups of a launch with so few tokens that it uses smaller ones (CombineGroup)
+  int grid = 0;          // workers (FinishGeometry)
   uint32_t queue_cap = 0;
 };
 
-// Slots of any task queue of a rank: at least every task one launch can publish there, so
-// that a slot is never reused within a launch.  Tile tasks of the rank's experts (FFN1 in one
-// queue, FFN2 in the other), COMBINE tasks (one per group of combine_group tokens), GATEFIX
+// Tasks that a launch of many tokens can publish on any queue of a rank: tile tasks of the rank's experts
+// (FFN1 in one queue, FFN2 in the other), COMBINE tasks (one per group of combine_group tokens), GATEFIX
 // tasks (two tokens each, every token in the worst case, rounded up per GATE tile), the GATED round,
 // and DISPATCH tasks (one per GATE tile of at least 32 tokens).
-inline uint64_t WorstCaseQueueTasks(const Geometry& g) {
+inline uint64_t ManyTokenQueueTasks(const Geometry& g) {
   const uint64_t rows_max = std::min<uint64_t>((uint64_t)g.max_tokens_sum * g.K, (uint64_t)g.El * g.cap_rows);
   const uint64_t mtiles = rows_max / FDMOE_TILE_M + g.El;
   const uint64_t tiles = mtiles * (uint64_t)std::max(g.I / FDMOE_TILE_N1, g.H / FDMOE_TILE_N2);
@@ -66,21 +66,32 @@ inline uint64_t WorstCaseQueueTasks(const Geometry& g) {
          (uint64_t)g.max_tokens_max / 2 + gate_tiles + 1;
 }
 
+// Every task that any launch can publish on a queue.  One of few tokens on one GPU has smaller COMBINE groups
+// (up to small_groups, CombineGroup) and GATE tiles of one token (up to one per worker, GateRows), each of which
+// may publish a GATEFIX task.
+inline uint64_t WorstCaseQueueTasks(const Geometry& g) {
+  const uint64_t fewer = g.world == 1 ? (uint64_t)std::min(g.max_tokens_max, g.grid) : 0;
+  return ManyTokenQueueTasks(g) + (uint64_t)g.small_groups + fewer;
+}
+
+// Slots of any queue: more than every task of a launch, so that a slot is never reused within one.  The slots
+// on top hold what launches of few tokens have more (two tasks per worker) and the self-tests' tasks.
 inline uint32_t QueueCapacity(const Geometry& g, int grid) {
-  return NextPow2(WorstCaseQueueTasks(g) + (uint64_t)grid + 2048);
+  return NextPow2(ManyTokenQueueTasks(g) + (uint64_t)grid + 2048);
 }
 
 // Derived sizes once the token bounds, the shape and combine_group are known: rows of a local expert's
 // buffer (an expert receives at most one row per token of any rank), m-tiles per expert, queue
 // capacity.  Returns false when the expert buffers would hold more rows than a dispatch word can
-// address (28 bits).
+// address (28 bits), or the queues fewer slots than tasks (more than 2048 workers).
 inline bool FinishGeometry(Geometry& g, int grid) {
   const uint64_t cap = AlignUp((size_t)std::max<int64_t>(g.max_tokens_sum, 1), FDMOE_TILE_M);
   if ((uint64_t)g.El * cap >= (1ull << 28)) return false;
   g.cap_rows = (int)cap;
   g.MT = g.cap_rows / FDMOE_TILE_M;
+  g.grid = grid;
   g.queue_cap = QueueCapacity(g, grid);
-  return true;
+  return g.queue_cap >= WorstCaseQueueTasks(g);
 }
 
 inline size_t CombineGroups(const Geometry& g) {

@@ -132,7 +132,7 @@ extern "C" int FlashMoeLaunchNoAlloc(const void* gateWeights, const void* ffn1Ex
   g.world = 1;
   g.max_tokens_local = g.max_tokens_max = std::max(tokensNum, 1);
   g.max_tokens_sum = g.max_tokens_max;
-  g.combine_group = 8;
+  g.combine_group = 8;  // at any token count: counters for smaller groups would take scratch that accepted calls do not have
   if (!FinishGeometry(g, d->grid)) return (int)cudaErrorInvalidValue;
   const ArenaLayout L = MakeLayout(g);
   // regions the launcher allocates separately follow the arena inside the same array

@@ -36,10 +36,31 @@ int main() {
           const size_t gates = ((size_t)t + gr - 1) / gr;
           CHECK(gr > 2 || gates <= (size_t)grid);
           const uint64_t tiles = ((uint64_t)t * g.K / FDMOE_TILE_M + g.El) * (g.H / FDMOE_TILE_N2);
-          CHECK(tiles + groups + (gr > 2 ? (uint64_t)t / 2 + gates : 0) + 1 <= g.queue_cap);
+          // (GATEFIX tasks: one per tile of one or two tokens, else two tokens each, rounded up per tile)
+          const uint64_t fix = gr <= 2 ? gates : (uint64_t)t / 2 + gates;
+          CHECK(tiles + groups + fix + 1 <= WorstCaseQueueTasks(g));
+          CHECK(WorstCaseQueueTasks(g) <= g.queue_cap);
+          // tiles that a caller may ask for: the same bound
+          for (int rows : {1, 2, 3, 32, 64, 128, 256}) {
+            CHECK(GateRowsFit(rows, t, grid, 1) == (rows == 2 || rows == 32 || rows == 64 || rows == 128 || (rows == 1 && t <= grid)));
+            CHECK(GateRowsFit(rows, t, grid, 2) == (rows == 32 || rows == 64 || rows == 128));
+            const uint64_t tl = ((uint64_t)t + rows - 1) / rows;
+            if (GateRowsFit(rows, t, grid, 1))
+              CHECK(tiles + groups + (rows <= 2 ? tl : (uint64_t)t / 2 + tl) + 1 <= WorstCaseQueueTasks(g));
+          }
         }
       }
     }
+  }
+  // wide FFN tasks: both sides of the line of three FFN1 tasks of 256 rows per worker
+  {
+    Geometry g;
+    g.H = 2048; g.I = 768; g.E = g.El = 128; g.K = 8;
+    CHECK(WideRows(g, 0, 148) == kNoWideRows);
+    CHECK(WideRows(g, 2367, 148) == kNoWideRows && WideRows(g, 2368, 148) == FDMOE_TILE_M);  // 73 and 74 m-tile pairs x 6
+    g.H = 4096; g.I = 1536;
+    CHECK(WideRows(g, 1183, 148) == kNoWideRows && WideRows(g, 1184, 148) == FDMOE_TILE_M);  // 36 and 37 x 12
+    CHECK(WideRows(g, 1 << 20, 1) == FDMOE_TILE_M);
   }
   if (failures) std::printf("%d checks failed\n", failures);
   return failures != 0;
