@@ -443,8 +443,8 @@ __device__ __forceinline__ FdmoeSlot next_task(const FdmoeParams& p, SmemCtl& sc
   uint32_t spins = 0;
   for (;;) {
     if (sc.abort) return exit_task();
-    // every word the decision rests on, asked for at once: one after the other they are five round trips to
-    // L2, 0.7 us each, before an idle worker sees its task
+    // every word the decision rests on, asked for at once instead of one round trip to L2 after another: 0.9 us
+    // less over the hand-overs of a launch of one token
     const int32_t n0 = (int32_t)ld_relaxed<S>(&ctl->q[0].avail), n1 = (int32_t)ld_relaxed<S>(&ctl->q[1].avail);
     const int32_t n2 = (int32_t)ld_relaxed<false>(&ctl->q[2].avail);
     const uint32_t gates = ld_relaxed<false>(&ctl->gate_next), closed = ld_relaxed<false>(&ctl->closed);
@@ -914,9 +914,9 @@ __device__ __noinline__ bool dispatch_task(const FdmoeParams& p, SmemCtl& sc, ui
 // output (bf16 x bf16 products are exact in fp32, so this equals the reference's `acc += a*b` bit for bit;
 // reference refGemm.h:16-27).  The stage holds up to three 64-column boxes of gate weights (TMA, 128-byte
 // swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7)); the token rows are fp32 and broadcast.
-// A dependent FMA every four cycles is the floor of this loop.  What could hold it up is unpacking (half
-// the FMA rate) and shared-memory reads, so the token rows are unpacked once per task and one thread
-// serves both tokens, which read and unpack a weight once.
+// Bound by the chain of dependent FMAs and the unpacking between them: 12.5 us at H = 2048.  To keep the rest small,
+// the token rows are unpacked once per task and one thread serves both tokens, which read and unpack a weight
+// once.
 template <bool Two>
 __device__ __forceinline__ void exact_logits(const uint8_t* stage, const float* xa, const float* xb, uint32_t e,
                                              uint32_t blocks, float& acc_a, float& acc_b) {
@@ -961,30 +961,75 @@ __device__ __forceinline__ TokenRow load_row(const FdmoeParams& p, uint32_t tok,
   return x;
 }
 
-// A nearly tied token of a GATE tile of one or two: the exact logits of the experts it may select, up to 32 of
-// them, one per lane (fp32 FMAs, k ascending, as exact_logits).  `rows` holds the token's row and behind it the
-// experts' gate rows, 16 bytes apart.  A chain of H dependent FMAs of four cycles is the floor.
-__device__ __forceinline__ float exact_logit(const uint8_t* rows, int H, uint32_t lane_row) {
-  const uint4* x = reinterpret_cast<const uint4*>(rows);
-  const uint4* w = reinterpret_cast<const uint4*>(rows + (size_t)H * 2 + (size_t)lane_row * (H * 2 + 16));
+// A nearly tied token of a GATE tile of one or two: the exact logits of the experts it may select, one per lane
+// (fp32 FMAs, k ascending, as exact_logits), from rows that are fp32 already.  Bound by the chain of H dependent FMAs:
+// 8.8 us at H = 2048, also with the operands read 16 steps ahead; unpacking bf16 rows in the loop took 13.
+__device__ __forceinline__ float exact_logit(const float4* x, const float4* w, int H) {
   float acc = 0.f;
 #pragma unroll 8
-  for (int c = 0; c < H / 8; ++c) {
-    const uint4 xv = x[c], wv = w[c];
-    acc = fmaf(bf16_lo(xv.x), bf16_lo(wv.x), acc);
-    acc = fmaf(bf16_hi(xv.x), bf16_hi(wv.x), acc);
-    acc = fmaf(bf16_lo(xv.y), bf16_lo(wv.y), acc);
-    acc = fmaf(bf16_hi(xv.y), bf16_hi(wv.y), acc);
-    acc = fmaf(bf16_lo(xv.z), bf16_lo(wv.z), acc);
-    acc = fmaf(bf16_hi(xv.z), bf16_hi(wv.z), acc);
-    acc = fmaf(bf16_lo(xv.w), bf16_lo(wv.w), acc);
-    acc = fmaf(bf16_hi(xv.w), bf16_hi(wv.w), acc);
+  for (int c = 0; c < H / 4; ++c) {
+    const float4 xv = x[c], wv = w[c];
+    acc = fmaf(xv.x, wv.x, acc);
+    acc = fmaf(xv.y, wv.y, acc);
+    acc = fmaf(xv.z, wv.z, acc);
+    acc = fmaf(xv.w, wv.w, acc);
   }
   return acc;
 }
-constexpr uint32_t kHalfStages = kStages / 2 * kStageBytes;  // what exact_logit's rows of one token may take
+// A row in the stages: H fp32 values, and 16 bytes so that the lanes' reads meet no bank twice.
+__device__ __forceinline__ uint32_t exact_row_bytes(int H) { return (uint32_t)H * 4u + 16u; }
+// Candidates whose rows fit the stages behind the token's.
 __device__ __forceinline__ uint32_t max_candidates(int H) {
-  return min(32u, (kHalfStages - (uint32_t)H * 2u) / ((uint32_t)H * 2u + 16u));
+  return min(31u, (uint32_t)(kStages * kStageBytes) / exact_row_bytes(H) - 1u);
+}
+__device__ __forceinline__ void store_unpacked(uint8_t* row, int piece, const uint4& v) {
+  float4* dst = reinterpret_cast<float4*>(row) + 2 * piece;
+  dst[0] = make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
+  dst[1] = make_float4(bf16_lo(v.z), bf16_hi(v.z), bf16_lo(v.w), bf16_hi(v.w));
+}
+// Leaves the exact logits of the `n` candidates of token `tok`, the tile's first or second (`t`), in sc.logits[t], for
+// the first warp of that half of the group, and none of the others.  Called by the whole group.
+__device__ __noinline__ void regate_tied(const FdmoeParams& p, SmemCtl& sc, uint8_t* stage, int etid, int t, uint32_t n,
+                                         uint32_t tok) {
+  const int H = p.H, lane = etid & 31;
+  const uint32_t rowb = exact_row_bytes(H);
+  if (t) epi_bar();  // (the first token's rows may lie where the second one's go)
+  // the token's row and the gate rows, as they are, into the upper halves of their places
+  for (uint32_t r = 0; r <= n; ++r) {
+    const uint4* src = r ? reinterpret_cast<const uint4*>(p.gate_w) + (size_t)sc.cand[t][r - 1u] * (H / 8)
+                         : reinterpret_cast<const uint4*>(p.x) + (size_t)tok * (H / 8);
+    for (int c = etid; c < H / 8; c += kEpiThreads) ptx::cp_async16(stage + r * rowb + H * 2 + c * 16, src + c);
+  }
+  ptx::cp_async_wait_all();
+  // unpacked in place, two rows and 4 KB of each at a time: every piece is read before anything is written over it
+  // (the first 256 pieces become bytes 0 to 8191, the next ones lie from byte 2 H + 4096 on, H being 2048 then at
+  // least; a thread reads its own copies)
+  for (uint32_t r0 = 0; r0 <= n; r0 += 2u) {
+    for (int c = etid; c - etid < H / 8; c += kEpiThreads) {
+      const bool in = c < H / 8;
+      const uint8_t* src = stage + H * 2 + (in ? c : 0) * 16;
+      const uint4 v0 = *reinterpret_cast<const uint4*>(src + min(r0, n) * rowb);
+      const uint4 v1 = *reinterpret_cast<const uint4*>(src + min(r0 + 1u, n) * rowb);
+      epi_bar();
+      if (in) {
+        store_unpacked(stage + r0 * rowb, c, v0);
+        if (r0 < n) store_unpacked(stage + (r0 + 1u) * rowb, c, v1);
+      }
+    }
+  }
+  epi_bar();
+  prof_mark(p, sc, etid, 33);
+  if (etid >> 5 == 4 * t) {
+    const uint32_t row = min((uint32_t)lane, n - 1u) + 1u;
+    const float acc = exact_logit(reinterpret_cast<const float4*>(stage),
+                                  reinterpret_cast<const float4*>(stage + row * rowb), H);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sc.logits[t][lane + 32 * i] = -INFINITY;
+    __syncwarp();
+    if ((uint32_t)lane < n) sc.logits[t][sc.cand[t][lane]] = acc;
+    __syncwarp();
+  }
+  prof_mark(p, sc, etid, 34);
 }
 constexpr uint32_t kManyTied = 0xffffffffu;  // more candidates than that: the token goes to a GATEFIX task
 
@@ -994,8 +1039,9 @@ constexpr uint32_t kManyTied = 0xffffffffu;  // more candidates than that: the t
 // `Check`: the logits are the tensor cores'.  A nearly tied token's K largest exact logits are among those of
 // the experts whose tensor-core logit is at most the gap below its K-th largest one; these are recomputed here,
 // with the gate rows in the stages, which are free while this task runs.  (A GATEFIX task instead costs
-// two queue hand-overs and all E logits; at 128 tokens of the 2048 x 768 shape two or three tokens are nearly tied
-// and the first FFN tile starts behind them.)  Called by the whole group, behind a barrier.
+// two queue hand-overs and all E logits, 28 us against 12, behind which the first FFN tile starts: at 128 tokens
+// of the 2048 x 768 shape, two or three of them nearly tied, the layer took 263 us with it and takes 246, at 48
+// tokens in fp32 251 and 244.)  Called by the whole group, behind a barrier.
 template <bool S, bool Check>
 __device__ __forceinline__ void route_tokens(const FdmoeParams& p, SmemCtl& sc, uint8_t* stage, int etid, int ewarp,
                                              int lane, uint32_t tok, bool live, bool two, const TokenRow& x) {
@@ -1029,32 +1075,11 @@ __device__ __forceinline__ void route_tokens(const FdmoeParams& p, SmemCtl& sc, 
     epi_bar();
     tie_a = sc.pre[0];
     tie_b = two ? sc.pre[1] : 0u;
-    const bool in_a = tie_a != 0u && tie_a != kManyTied, in_b = tie_b != 0u && tie_b != kManyTied;
-    if (in_a || in_b) {
-      const uint32_t n = half ? tie_b : tie_a;
-      const bool exact = half ? in_b : in_a;
-      uint8_t* rows = stage + half * kHalfStages;
-      if (exact) {
-        const uint4* gate = reinterpret_cast<const uint4*>(p.gate_w);
-        for (uint32_t r = 0; r < n; ++r)
-          for (int c = e; c < H / 8; c += 128)
-            ptx::cp_async16(rows + (size_t)H * 2 + (size_t)r * (H * 2 + 16) + c * 16,
-                            gate + (size_t)sc.cand[half][r] * (H / 8) + c);
-#pragma unroll
-        for (int i = 0; i < FDMOE_MAX_HIDDEN / 8 / 128; ++i)
-          if (e + i * 128 < H / 8) reinterpret_cast<uint4*>(rows)[e + i * 128] = x.v[i];
-        ptx::cp_async_wait_all();
-      }
-      epi_bar();
-      if (mine && exact) {
-        const float acc = exact_logit(rows, H, min((uint32_t)lane, n - 1u));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) sc.logits[half][lane + 32 * i] = -INFINITY;
-        __syncwarp();
-        if ((uint32_t)lane < n) sc.logits[half][sc.cand[half][lane]] = acc;
-        __syncwarp();
-        topk_warp<1>(sc.logits[half], 128, E, K, lane, topv, topi);
-      }
+    for (int t = 0; t < 2; ++t) {
+      const uint32_t n = t ? tie_b : tie_a;
+      if (n == 0u || n == kManyTied) continue;
+      regate_tied(p, sc, stage, etid, t, n, tok - (uint32_t)half + (uint32_t)t);
+      if (mine && half == t) topk_warp<1>(sc.logits[half], 128, E, K, lane, topv, topi);
     }
   }
   const float myv = topv[0];
@@ -1139,11 +1164,12 @@ __device__ __forceinline__ void route_tokens(const FdmoeParams& p, SmemCtl& sc, 
 
 // Epilogue of a GATE tile of one or two tokens (launches of few tokens on one GPU, see GateRows): the tile's
 // MMAs are those of a larger tile, so a token's logits, and with them its routing weights, have the same bits
-// at any number of tokens.  The task sends the rows itself, without a DISPATCH task.
+// at any number of tokens.  The task sends the rows itself, without a DISPATCH task.  Bound by latency: 9 us
+// for the gate weights (512 KB per worker at H = 2048, from L2), 3 for top-k and reservation, 4 for the rows.
 template <bool S>
 __device__ __noinline__ void gate_few_epilogue(const FdmoeParams& p, SmemCtl& sc, uint8_t* stage, uint32_t taddr,
-                                               uint64_t* tmem_empty_bar, int q, int h, int lane, int etid, int ewarp,
-                                               uint32_t tile) {
+                                               uint64_t* tmem_empty_bar, int etid, uint32_t tile) {
+  const int lane = etid & 31, ewarp = etid >> 5, q = ewarp & 3, h = ewarp >> 2;
   const uint32_t t0 = tile * (uint32_t)p.gate_rows;
   const bool two = p.gate_rows == 2 && t0 + 1u < (uint32_t)p.T;
   const uint32_t half = (uint32_t)etid >> 7;
@@ -1440,14 +1466,14 @@ __device__ __forceinline__ void ffn2_epilogue(SmemCtl& sc, uint32_t taddr, uint6
 }
 
 // A (half) tile of up to 64 rows is computed transposed: the weights are the M operand, two blocks of 128,
-// and the rows the N operand, in steps of 16.  As M operand the rows are padded to 128.  What that costs is
-// power: the board's limit holds this kernel's clock down (1.3 GHz of 1.965 measured inside back-to-back
-// launches of 128 tokens, 1.2 to 1.45 GHz at 4096), and MMAs on rows that do not exist take their share of
-// it also where memory sets the pace.  The line is the one up to which rows are loaded in boxes of 16; at 64
-// rows the transposed form has half the MMA cycles.  With peers the other form stays, whose stores over
-// NVLink are whole lines.  Whole layer, padded and transposed: 4096 x 1536 shape at 64 tokens 869 and
-// 780 us, at 2048 tokens 1237 and 1156; 2048 x 768 shape at 16, 128, 333, 4096 tokens 175 and 171, 268 and
-// 249, 302 and 289, 582 and 576.
+// and the rows the N operand, in steps of 16.  As M operand the rows are padded to 128, and the tensor cores
+// work on rows that do not exist.  That this costs time also where memory sets the pace is measured, why is
+// not (power may be a part of it: the clock seen inside back-to-back launches is 1.2 to 1.45 GHz of 1.965).
+// The line is the one up to which rows are loaded in boxes of 16; at 64 rows the transposed form has half
+// the MMA cycles.  With peers the other form stays, whose stores over NVLink are whole lines (the transposed form
+// has not been measured there).  Whole layer, padded and transposed: 4096 x 1536 shape at 64 tokens 834 and
+// 782 us, at 2048 tokens 1250 and 1101; 2048 x 768 shape at 16, 128, 333, 4096 tokens 168 and 167, 262 and
+// 256, 295 and 285, 555 and 527.
 // Block b of the weights has its accumulator at column b * kBlockCols; lanes are weight rows.
 constexpr uint32_t kBlockCols = 64;
 template <bool S>
@@ -1547,8 +1573,9 @@ __device__ __forceinline__ uint32_t gate_kblocks_per_stage(bool is_gate, int gat
 // Brings `rows` (1..128) rows of an expert's buffer, one k-block wide, into a stage: in boxes of 16 rows
 // up to 64, else in one box of 128.  The stage's other rows keep what was there: they only reach
 // accumulator rows that nobody reads.  In a decode batch an expert holds a handful of rows, and a box of
-// 128 is a third of all operand bytes, most of it from DRAM since nothing ever wrote it.  Whole layer at 128
-// tokens of the 2048 x 768 shape: 294 us with boxes of 128, 288 us so; at 333 tokens 300 and 296 us.
+// 128 is a third of all operand bytes, most of it from DRAM since nothing ever wrote it.  Whole layer of the
+// 2048 x 768 shape with boxes of 128 and so: 16 tokens 174.7 and 166.7 us, 128 tokens 266 and 256, 333 tokens
+// 295 and 285.
 __device__ __forceinline__ uint32_t row_load_bytes(uint32_t rows) {
   return rows > 64u ? (uint32_t)kStageA : ((rows + 15u) / 16u) * (uint32_t)(FDMOE_ROW_BOX * FDMOE_TILE_K * 2);
 }
@@ -2040,8 +2067,7 @@ moe_persistent_kernel(const __grid_constant__ FdmoeParams p) {
         if (p.prof && etid == 0) pt1 = prof_now();
         ptx::tcgen05_fence_after();
         if (few_gated)
-          gate_few_epilogue<S>(task_params(sc), sc, stage, tmem_base + acc * kAccCols, &sc.tmem_empty[acc], q, h, lane, etid,
-                               ewarp, j);
+          gate_few_epilogue<S>(task_params(sc), sc, stage, tmem_base + acc * kAccCols, &sc.tmem_empty[acc], etid, j);
         else
           gate_epilogue<S>(task_params(sc), sc, tmem_base + acc * kAccCols, &sc.tmem_empty[acc], q, h, lane, etid, ewarp, j);
       } else if (kind == FDMOE_TASK_DISPATCH) {
