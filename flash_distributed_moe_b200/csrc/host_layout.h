@@ -100,7 +100,8 @@ inline size_t CombineGroups(const Geometry& g) {
 
 // Tokens per COMBINE task of a launch on one GPU: as many as give every worker one task, `most` at most.
 // The groups of a decode batch all complete at the end, and nothing is left to overlap them with.
-// Whole layer at 128 tokens of the 2048 x 768 shape: 262 us in groups of 8, 258 us in groups of one.
+// Whole layer of the 2048 x 768 shape on 148 SMs in groups of 8 and so: 16 tokens 170.5 and 166.7 us, 128 tokens
+// 260 and 256, 333 tokens 287.6 and 285, 592 tokens 298 and 295.
 inline int CombineGroup(int tokens, int grid, int most) {
   int g = 1;
   while (g < most && tokens > g * grid) g *= 2;
@@ -142,9 +143,9 @@ inline ArenaLayout MakeLayout(const Geometry& g) {
 // Experts with more rows than this get wide FFN tasks (FDMOE_TILE_WIDE) in a launch on one GPU.  Wide tasks are
 // twice as long, and going from narrow to wide stages drains the pipeline, so a launch uses them only if
 // there are about three wide FFN1 tasks per worker.  Whole layer on 148 SMs, narrow only and wide from 129
-// rows on: 16 experts of 4096 x 1536 at 400 tokens (1.0 tasks per worker) 265 and 299 us, at 700 (1.8) 325
-// and 358, at 1300 (3.3) 503 and 484; 2048 x 768 shape at 1800 tokens (2.3) 332 and 350, at 2048 (2.6) 347
-// and 366, at 2500 (3.2) 402 and 396; 4096 x 1536 shape at 2048 tokens (5.2) 1184 and 1115.
+// rows on: 16 experts of 4096 x 1536 at 400 tokens (1.0 tasks per worker) 268 and 303 us, at 700 (1.8) 329
+// and 362, at 1300 (3.3) 499 and 497; 2048 x 768 shape at 1800 tokens (2.3) 350 and 355, at 2048 (2.6) 355
+// and 369, at 2500 (3.2) 412 and 399; 4096 x 1536 shape at 2048 tokens (5.2) 1160 and 1078.
 constexpr int kNoWideRows = 1 << 30;
 inline int WideRows(const Geometry& g, int tokens, int grid) {
   const uint64_t tasks = (uint64_t)tokens * g.K / (2 * FDMOE_TILE_M) * (g.I / FDMOE_TILE_N1);
@@ -154,7 +155,10 @@ inline int WideRows(const Geometry& g, int tokens, int grid) {
 // Tokens per GATE tile of a launch on one GPU.  32, 64 or 128: the smallest that still gives every SM at most
 // one tile, so that the gate phase spreads over as many SMs as possible.  1 or 2: the tile's task sends its
 // tokens' rows too, which saves a small launch the separate DISPATCH tasks, as long as one wave of
-// workers does it.
+// workers does it.  Whole layer on 148 SMs, one token per tile / two / 32: 2048 x 768 shape at 128 tokens 256 /
+// 256 / 276 us, 148 tokens 256 / 257 / 276, 296 tokens - / 263 / 282, 592 tokens - / 292 / 295; 16 experts of
+// 4096 x 1536 at 64 tokens 174 / 174 / 225, 148 tokens 184 / 185 / 233, 296 tokens - / 230 / 258, 592 tokens
+// - / 316 / 330; 128 of them at 148 tokens 807 / 812 / 838, 296 tokens - / 826 / 856, 592 tokens - / 905 / 888.
 inline int GateRows(int tokens, int grid) {
   if (tokens <= grid) return 1;
   if (tokens <= 2 * grid) return 2;

@@ -56,7 +56,7 @@ enum {
 // whether it is wide.  A wide task runs two m-tiles of an expert against each block of weights, which
 // brings 64 KB of operands into shared memory for what costs two narrow ones 96 KB.  On one GPU an
 // expert's tasks are wide from 129 rows on, where there is a second m-tile, if the launch has enough of
-// them (WideRows).  Whole layer, narrow and wide: 16384 tokens of the 2048 x 768 shape 1560 and 1513 us.
+// them (WideRows).  Whole layer, narrow and wide: 8192 tokens of the 2048 x 768 shape 794 and 781 us.
 // With peers they stay narrow: a wide task holds both accumulators through its epilogue, whose stores
 // cross NVLink there.
 enum {
