@@ -1039,9 +1039,9 @@ constexpr uint32_t kManyTied = 0xffffffffu;  // more candidates than that: the t
 // `Check`: the logits are the tensor cores'.  A nearly tied token's K largest exact logits are among those of
 // the experts whose tensor-core logit is at most the gap below its K-th largest one; these are recomputed here,
 // with the gate rows in the stages, which are free while this task runs.  (A GATEFIX task instead costs
-// two queue hand-overs and all E logits, 28 us against 12, behind which the first FFN tile starts: at 128 tokens
-// of the 2048 x 768 shape, two or three of them nearly tied, the layer took 263 us with it and takes 246, at 48
-// tokens in fp32 251 and 244.)  Called by the whole group, behind a barrier.
+// two queue hand-overs and all E logits: at 128 tokens of the 2048 x 768 shape, of which two or three are nearly tied
+// as a rule, the first FFN tile starts at 47 us with it and at 38 so, the layer takes 263 us with it and 246 to
+// 256 so.  Without a nearly tied token it is 25 and 240 to 243.)  Called by the whole group, behind a barrier.
 template <bool S, bool Check>
 __device__ __forceinline__ void route_tokens(const FdmoeParams& p, SmemCtl& sc, uint8_t* stage, int etid, int ewarp,
                                              int lane, uint32_t tok, bool live, bool two, const TokenRow& x) {
